@@ -351,25 +351,67 @@ int alloc_records(lemc_ctx* c) {
 
 int setup_tc(lemc_ctx* c, int force_splits = 0);
 
-// SIMT job list: same-sector Gram tiles {ONE, R2, R4} and, for every ordered
-// pair of sectors (diagonal pairs included), cross tiles {USER, COS_l, SIN_l}
-// with l = |dL_j - dL_i| (cos/sin disabled unless l is a probe).
+// Row chunks of a sector of `dim` states for the SIMT tiles: 32 rows each, the
+// rest in the smallest of 8, 16 or 32 that holds it.
+std::vector<std::pair<int, int>> simt_chunks(int dim) {
+  std::vector<std::pair<int, int>> out;  // (first row, tile extent)
+  for (int r = 0; r < dim; r += 32) {
+    const int n = dim - r;
+    out.push_back({r, n > 16 ? 32 : n > 8 ? 16 : 8});
+  }
+  return out;
+}
+
+// Tiles of the block (sector i) x (sector j): `off` is the offset of that block
+// in the output, `off_t` that of the transposed one, which the same jobs fill
+// (i == j: off == off_t, and only one of two transposed tiles is listed).
+void simt_jobs(const lemc_ctx* c, int i, int j, int off, int off_t, const int (&plane)[3], int buf,
+               std::vector<GramJob>* jobs) {
+  const int di = c->basis.sector_dim[i], dj = c->basis.sector_dim[j];
+  const auto ci = simt_chunks(di), cj = simt_chunks(dj);
+  for (size_t x = 0; x < ci.size(); ++x)
+    for (size_t y = i == j ? x : 0; y < cj.size(); ++y) {
+      const bool diag = i == j && x == y;
+      GramJob jb{};
+      const bool swap = ci[x].second > cj[y].second;  // the kernel's shapes have ta <= tb
+      jb.row_a = c->sec_row[swap ? j : i];
+      jb.Da = swap ? dj : di;
+      jb.row_b = c->sec_row[swap ? i : j];
+      jb.Db = swap ? di : dj;
+      jb.a0 = swap ? cj[y].first : ci[x].first;
+      jb.b0 = swap ? ci[x].first : cj[y].first;
+      jb.ta = swap ? cj[y].second : ci[x].second;
+      jb.tb = swap ? ci[x].second : cj[y].second;
+      for (int h = 0; h < 3; ++h) jb.plane[h] = plane[h];
+      jb.buf = buf;
+      jb.out = swap ? off_t : off;
+      jb.mirror = diag ? -1 : swap ? off : off_t;
+      jobs->push_back(jb);
+    }
+}
+
+// SIMT job list: same-sector Gram tiles {ONE, R2, R4} and, for every pair of
+// sectors (diagonal pairs included), cross tiles {USER, COS_l, SIN_l} with
+// l = |dL_j - dL_i| (cos/sin disabled unless l is a probe); the jobs of a pair
+// i < j fill (i, j) and (j, i).
 int build_jobs(lemc_ctx* c) {
   const auto& sec = c->basis.sectors;
+  const int ns = int(sec.size());
   std::vector<GramJob> jobs;
-  for (size_t s = 0; s < sec.size(); ++s) {
-    const int dim = c->basis.sector_dim[s];
-    for (int a0 = 0; a0 < dim; a0 += 16)
-      for (int b0 = 0; b0 < dim; b0 += 16)
-        jobs.push_back({c->sec_row[s], dim, c->sec_row[s], dim, a0, b0,
-                        {LEMC_W_ONE, LEMC_W_R2, LEMC_W_R4}, 0, c->sec_goff[s]});
-  }
+  for (int s = 0; s < ns; ++s)
+    simt_jobs(c, s, s, c->sec_goff[s], c->sec_goff[s], {LEMC_W_ONE, LEMC_W_R2, LEMC_W_R4}, 0, &jobs);
   c->n_gram_jobs = int(jobs.size());
   c->cross_pairs.clear();
   c->cross_off.clear();
   size_t coff = 0;
-  for (size_t i = 0; i < sec.size(); ++i)
-    for (size_t j = 0; j < sec.size(); ++j) {
+  for (int i = 0; i < ns; ++i)
+    for (int j = 0; j < ns; ++j) {
+      c->cross_pairs.push_back({i, j});
+      c->cross_off.push_back(coff);
+      coff += size_t(c->basis.sector_dim[i]) * c->basis.sector_dim[j];
+    }
+  for (int i = 0; i < ns; ++i)
+    for (int j = i; j < ns; ++j) {
       const int l = std::abs(sec[j] - sec[i]);
       int pc = -1, ps = -1;
       for (size_t q = 0; q < c->probes.size(); ++q)
@@ -377,14 +419,8 @@ int build_jobs(lemc_ctx* c) {
           pc = LEMC_W_PROBE0 + 2 * int(q);
           ps = pc + 1;
         }
-      c->cross_pairs.push_back({int(i), int(j)});
-      c->cross_off.push_back(coff);
-      const int da = c->basis.sector_dim[i], db = c->basis.sector_dim[j];
-      for (int a0 = 0; a0 < da; a0 += 16)
-        for (int b0 = 0; b0 < db; b0 += 16)
-          jobs.push_back({c->sec_row[i], da, c->sec_row[j], db, a0, b0, {LEMC_W_USER, pc, ps}, 1,
-                          int(coff)});
-      coff += size_t(da) * db;
+      simt_jobs(c, i, j, int(c->cross_off[size_t(i) * ns + j]), int(c->cross_off[size_t(j) * ns + i]),
+                {LEMC_W_USER, pc, ps}, 1, &jobs);
     }
   c->cross_plane = coff;
   c->n_cross_jobs = int(jobs.size()) - c->n_gram_jobs;
@@ -489,9 +525,8 @@ int gram_step(lemc_ctx* c, const float* V, const float* rec_w, int ldw, int W, i
   const bool cross =
       c->n_cross_jobs > 0 && (c->hooked || c->multipole_k > 0 || !c->probes.empty());
   if (mode == LEMC_GRAM_FP64) {
-    const int splits = std::max(1, std::min(64, W / 1024));
     return launch_gram_simt(V, c->Wpad, rec_w, ldw, W, c->jobs.p,
-                            c->n_gram_jobs + (cross ? c->n_cross_jobs : 0), splits, c->gram.p,
+                            c->n_gram_jobs + (cross ? c->n_cross_jobs : 0), c->gram.p,
                             c->gram_plane, c->cross.p, c->cross_plane, c->stream);
   }
   if (c->tc_tiles.empty()) LEMC_TRY(setup_tc(c, c->gram_splits));
@@ -501,9 +536,8 @@ int gram_step(lemc_ctx* c, const float* V, const float* rec_w, int ldw, int W, i
   if (s != LEMC_OK) return s;
   // cross-sector planes (user potential, cos/sin probes): FP64 path
   if (cross) {
-    const int splits = std::max(1, std::min(64, W / 1024));
     s = launch_gram_simt(V, c->Wpad, rec_w, ldw, W, c->jobs.p + c->n_gram_jobs, c->n_cross_jobs,
-                         splits, c->gram.p, c->gram_plane, c->cross.p, c->cross_plane, c->stream);
+                         c->gram.p, c->gram_plane, c->cross.p, c->cross_plane, c->stream);
   }
   return s;
 }

@@ -17,80 +17,209 @@
 namespace lemc {
 namespace {
 
-constexpr int TS = 16;     // 16 x 16 output tile
-constexpr int CH = 64;     // walkers per staged chunk
+constexpr int kGramThreads = 256;
+constexpr size_t kGramSmem = 40 * 1024;
 
-__global__ void __launch_bounds__(256)
-gram_simt_kernel(const float* __restrict__ V, int ldv, const float* __restrict__ rec_w, int ldw,
-                 int W,
-                 const GramJob* __restrict__ jobs, int n_splits, double* __restrict__ out0,
-                 size_t plane0, double* __restrict__ out1, size_t plane1) {
-  // plane[h] < 0 disables sum h
-  const GramJob jb = jobs[blockIdx.x];
-  const int split = blockIdx.y;
-  const int per = (W + n_splits - 1) / n_splits;
-  const int wbeg = split * per;
-  const int wend = min(W, wbeg + per);
+// Tile shapes (rows a x rows b).  A block of 256 threads computes one tile of
+// one walker range; a thread owns 2 x 2 outputs (24 FP64 sums), so a tile takes
+// TA TB / 4 threads and the block holds NG = 1024 / (TA TB) groups that share
+// each staged chunk of walkers, summed at the end.
+//
+// Bound: the FP64 pipe (64 FMA/cycle/SM).  A (pair, walker) costs 10 FMAs: 4
+// for conj(a) b, 6 for the three weighted sums (folding the weights into one
+// operand first would cost 12).  The staged values are widened to FP64 once per
+// chunk; widening inside the product loop, seven conversions for every 10 FMAs
+// at a quarter of their rate, and one output per thread held the previous
+// 16 x 16 form at 5 % of the pipe.  The small shapes keep the padding of small
+// sectors low and spread their walkers over more blocks.
+//
+// Measured (B200): cross planes of 526 states at 65536 walkers (N=100, dL
+// 0,2..16) @CROSS@; 29 states (N=8, dL 1..6) at 4096 walkers @SMALL@.
+template <int TA, int TB>
+struct Tile {
+  static constexpr int TX = TB / 2, TY = TA / 2;  // threads: tx over b, ty over a
+  static constexpr int TPG = TX * TY;
+  static constexpr int NG = kGramThreads / TPG;
+  static constexpr int CH = TA == 8 ? (TB == 8 ? 128 : TB == 16 ? 64 : 32) : (TB == 16 ? 64 : 32);
+  static constexpr int SA = TA + 1, SB = TB + 1;  // double2 row strides per walker
+  static constexpr int NF = 2 * (TA + TB) * CH / kGramThreads;  // staged floats per thread
+  static constexpr size_t kStage = sizeof(double2) * CH * (SA + SB) + sizeof(double) * 3 * CH;
+  static constexpr size_t kReduce = NG > 1 ? sizeof(double) * (NG / 2) * TPG * 24 : 0;
+  static_assert(NF * kGramThreads == 2 * (TA + TB) * CH && CH % 32 == 0 && CH % NG == 0, "tile shape");
+  static_assert(kStage <= kGramSmem && kReduce <= kGramSmem, "tile shape");
+};
 
-  __shared__ float are[TS][CH + 1], aim[TS][CH + 1], bre[TS][CH + 1], bim[TS][CH + 1];
-  __shared__ float wt[3][CH];
+// NW = 3: all three weight planes; NW = 1: only the first (the job's others are off)
+template <int TA, int TB, int NW>
+__device__ __forceinline__ void gram_tile(const float* __restrict__ V, int ldv,
+                                          const float* __restrict__ rec_w, int ldw, int wbeg,
+                                          int wend, const GramJob& jb, double* __restrict__ out,
+                                          size_t plane, unsigned char* smem) {
+  using T = Tile<TA, TB>;
+  double2* sa = reinterpret_cast<double2*>(smem);      // [CH][SA]
+  double2* sb = sa + T::CH * T::SA;                    // [CH][SB]
+  double* wt = reinterpret_cast<double*>(sb + T::CH * T::SB);  // [3][CH]
+  const int tid = threadIdx.x;
+  const int g = tid / T::TPG, tg = tid % T::TPG;
+  const int tx = tg % T::TX, ty = tg / T::TX;
 
-  const int tx = threadIdx.x % TS, ty = threadIdx.x / TS;
-  const int a = jb.a0 + ty, b = jb.b0 + tx;
-  double acc[6] = {0, 0, 0, 0, 0, 0};
-
-  for (int c0 = wbeg; c0 < wend; c0 += CH) {
-    for (int e = threadIdx.x; e < TS * CH; e += blockDim.x) {
-      const int r = e / CH, s = e % CH;
+  // staged element e = it * 256 + tid: walker e % CH, tile row e / CH in the
+  // order Re a, Im a, Re b, Im b (a warp reads 32 consecutive walkers of a row)
+  float pf[T::NF];
+  float pw[3] = {0.f, 0.f, 0.f};
+  auto fetch = [&](int c0) {
+#pragma unroll
+    for (int it = 0; it < T::NF; ++it) {
+      const int e = it * kGramThreads + tid;
+      const int s = e % T::CH, q = e / T::CH;
+      const bool isb = q >= 2 * TA;
+      const int t = isb ? q - 2 * TA : q;
+      const int tw = isb ? TB : TA;
+      const int r = (isb ? jb.b0 : jb.a0) + (t >= tw ? t - tw : t);
+      const int dim = isb ? jb.Db : jb.Da;
+      const int row = (isb ? jb.row_b : jb.row_a) + (t >= tw ? dim : 0) + r;
       const int wi = c0 + s;
-      const bool ok = wi < wend;
-      const int ra = jb.a0 + r, rb = jb.b0 + r;
-      are[r][s] = (ok && ra < jb.Da) ? V[(size_t)(jb.row_a + ra) * ldv + wi] : 0.f;
-      aim[r][s] = (ok && ra < jb.Da) ? V[(size_t)(jb.row_a + jb.Da + ra) * ldv + wi] : 0.f;
-      bre[r][s] = (ok && rb < jb.Db) ? V[(size_t)(jb.row_b + rb) * ldv + wi] : 0.f;
-      bim[r][s] = (ok && rb < jb.Db) ? V[(size_t)(jb.row_b + jb.Db + rb) * ldv + wi] : 0.f;
+      pf[it] = (wi < wend && r < dim) ? V[(size_t)row * ldv + wi] : 0.f;
     }
-    for (int e = threadIdx.x; e < 3 * CH; e += blockDim.x) {
-      const int h = e / CH, s = e % CH;
-      const int wi = c0 + s;
-      float v = 0.f;
-      const int pl = jb.plane[h];
-      if (wi < wend && pl >= 0) {
-        const float one = rec_w[(size_t)LEMC_W_ONE * ldw + wi];
-        v = (pl == LEMC_W_ONE) ? one : one * rec_w[(size_t)pl * ldw + wi];
+    if (tid < T::CH) {
+      const int wi = c0 + tid;
+      const float one = wi < wend ? rec_w[(size_t)LEMC_W_ONE * ldw + wi] : 0.f;
+#pragma unroll
+      for (int h = 0; h < NW; ++h) {
+        const int pl = jb.plane[h];
+        pw[h] = 0.f;
+        if (wi < wend && pl >= 0) pw[h] = pl == LEMC_W_ONE ? one : one * rec_w[(size_t)pl * ldw + wi];
       }
-      wt[h][s] = v;
     }
-    __syncthreads();
-#pragma unroll 4
-    for (int s = 0; s < CH; ++s) {
-      const double ar = are[ty][s], ai = aim[ty][s];
-      const double br = bre[tx][s], bi = bim[tx][s];
-      const double pr = ar * br + ai * bi;  // conj(a) * b
-      const double pi = ar * bi - ai * br;
-      const double w0 = wt[0][s], w1 = wt[1][s], w2 = wt[2][s];
-      acc[0] += w0 * pr;
-      acc[1] += w0 * pi;
-      acc[2] += w1 * pr;
-      acc[3] += w1 * pi;
-      acc[4] += w2 * pr;
-      acc[5] += w2 * pi;
+  };
+  auto stage = [&]() {
+    double* da = reinterpret_cast<double*>(sa);
+    double* db = reinterpret_cast<double*>(sb);
+#pragma unroll
+    for (int it = 0; it < T::NF; ++it) {
+      const int e = it * kGramThreads + tid;
+      const int s = e % T::CH, q = e / T::CH;
+      if (q < 2 * TA)
+        da[2 * (s * T::SA + (q % TA)) + (q / TA)] = double(pf[it]);
+      else
+        db[2 * (s * T::SB + ((q - 2 * TA) % TB)) + (q - 2 * TA) / TB] = double(pf[it]);
     }
+    if (tid < T::CH) {
+#pragma unroll
+      for (int h = 0; h < NW; ++h) wt[h * T::CH + tid] = double(pw[h]);
+    }
+  };
+
+  double2 acc[NW][2][2];
+#pragma unroll
+  for (int h = 0; h < NW; ++h)
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) acc[h][i][j] = make_double2(0.0, 0.0);
+
+  fetch(wbeg);
+  for (int c0 = wbeg; c0 < wend; c0 += T::CH) {
+    __syncthreads();  // the previous chunk is consumed
+    stage();
     __syncthreads();
+    if (c0 + T::CH < wend) fetch(c0 + T::CH);  // lands while this chunk is summed
+#pragma unroll 2
+    for (int s = g; s < T::CH; s += T::NG) {
+      double2 a[2], b[2];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        a[i] = sa[s * T::SA + ty + i * T::TY];
+        b[i] = sb[s * T::SB + tx + i * T::TX];
+      }
+      double w[NW];
+#pragma unroll
+      for (int h = 0; h < NW; ++h) w[h] = wt[h * T::CH + s];
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const double pr = a[i].x * b[j].x + a[i].y * b[j].y;  // conj(a) b
+          const double pi = a[i].x * b[j].y - a[i].y * b[j].x;
+#pragma unroll
+          for (int h = 0; h < NW; ++h) {
+            acc[h][i][j].x += w[h] * pr;
+            acc[h][i][j].y += w[h] * pi;
+          }
+        }
+    }
   }
-  if (a < jb.Da && b < jb.Db) {
-    // three weight planes, each `plane` complex entries apart
-    double* out = (jb.buf == 0) ? out0 : out1;
-    const size_t plane = (jb.buf == 0) ? plane0 : plane1;
-    if (!out) return;
-    const size_t idx = 2 * ((size_t)jb.out + (size_t)a * jb.Db + b);
-    atomicAdd(out + idx, acc[0]);
-    atomicAdd(out + idx + 1, acc[1]);
-    atomicAdd(out + idx + 2 * plane, acc[2]);
-    atomicAdd(out + idx + 2 * plane + 1, acc[3]);
-    atomicAdd(out + idx + 4 * plane, acc[4]);
-    atomicAdd(out + idx + 4 * plane + 1, acc[5]);
+  // fold the NG walker groups into group 0
+  if constexpr (T::NG > 1) {
+    double2* red = reinterpret_cast<double2*>(smem);
+    constexpr int kV = NW * 4;
+#pragma unroll
+    for (int off = T::NG / 2; off > 0; off >>= 1) {
+      __syncthreads();
+      if (g >= off && g < 2 * off) {
+#pragma unroll
+        for (int v = 0; v < kV; ++v)
+          red[v * (off * T::TPG) + (g - off) * T::TPG + tg] = acc[v >> 2][(v >> 1) & 1][v & 1];
+      }
+      __syncthreads();
+      if (g < off) {
+#pragma unroll
+        for (int v = 0; v < kV; ++v) {
+          const double2 o = red[v * (off * T::TPG) + g * T::TPG + tg];
+          acc[v >> 2][(v >> 1) & 1][v & 1].x += o.x;
+          acc[v >> 2][(v >> 1) & 1][v & 1].y += o.y;
+        }
+      }
+    }
+    if (g > 0) return;
   }
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int a = jb.a0 + ty + i * T::TY, b = jb.b0 + tx + j * T::TX;
+      if (a >= jb.Da || b >= jb.Db) continue;
+      const size_t o = 2 * ((size_t)jb.out + (size_t)a * jb.Db + b);
+      const size_t ot = 2 * ((size_t)jb.mirror + (size_t)b * jb.Da + a);
+#pragma unroll
+      for (int h = 0; h < NW; ++h) {
+        atomicAdd(out + o + 2 * plane * h, acc[h][i][j].x);
+        atomicAdd(out + o + 2 * plane * h + 1, acc[h][i][j].y);
+        if (jb.mirror >= 0) {  // the transposed block: conj of the same sum (real weights)
+          atomicAdd(out + ot + 2 * plane * h, acc[h][i][j].x);
+          atomicAdd(out + ot + 2 * plane * h + 1, -acc[h][i][j].y);
+        }
+      }
+    }
+}
+
+__global__ void __launch_bounds__(kGramThreads, 2)
+gram_simt_kernel(const float* __restrict__ V, int ldv, const float* __restrict__ rec_w, int ldw,
+                 int W, int per, const GramJob* __restrict__ jobs, double* __restrict__ out0,
+                 size_t plane0, double* __restrict__ out1, size_t plane1) {
+  __shared__ __align__(16) unsigned char smem[kGramSmem];
+  const GramJob jb = jobs[blockIdx.x];
+  const int wbeg = blockIdx.y * per;
+  const int wend = min(W, wbeg + per);
+  double* out = jb.buf == 0 ? out0 : out1;
+  const size_t plane = jb.buf == 0 ? plane0 : plane1;
+  if (!out || wbeg >= wend) return;
+  const bool one = jb.plane[1] < 0 && jb.plane[2] < 0;
+#define LEMC_TILE(A, B)                                                                   \
+  if (one)                                                                                \
+    gram_tile<A, B, 1>(V, ldv, rec_w, ldw, wbeg, wend, jb, out, plane, smem);             \
+  else                                                                                    \
+    gram_tile<A, B, 3>(V, ldv, rec_w, ldw, wbeg, wend, jb, out, plane, smem);             \
+  break
+  switch (jb.ta * 64 + jb.tb) {
+    case 8 * 64 + 8: LEMC_TILE(8, 8);
+    case 8 * 64 + 16: LEMC_TILE(8, 16);
+    case 8 * 64 + 32: LEMC_TILE(8, 32);
+    case 16 * 64 + 16: LEMC_TILE(16, 16);
+    case 16 * 64 + 32: LEMC_TILE(16, 32);
+    case 32 * 64 + 32: LEMC_TILE(32, 32);
+  }
+#undef LEMC_TILE
 }
 
 // Row sums of the reference estimator.  Block (row a, 32-column tile);
@@ -159,12 +288,20 @@ row_accumulate_kernel(const float* __restrict__ V, int ldv, const float* __restr
 }  // namespace
 
 int launch_gram_simt(const float* V, int ldv, const float* rec_w, int ldw, int W, const GramJob* jobs,
-                     int n_jobs, int n_splits, double* out0, size_t plane0, double* out1,
-                     size_t plane1, cudaStream_t st) {
+                     int n_jobs, double* out0, size_t plane0, double* out1, size_t plane1,
+                     cudaStream_t st) {
   if (n_jobs <= 0) return LEMC_OK;
-  dim3 grid(n_jobs, n_splits);
-  gram_simt_kernel<<<grid, 256, 0, st>>>(V, ldv, rec_w, ldw, W, jobs, n_splits, out0, plane0, out1,
-                                         plane1);
+  // Walker split: about sixteen blocks for each of the 2 x 148 resident slots, so
+  // the last wave is a small share (526 states:
+  // 9.2 ms; with six blocks a slot 9.9 ms), in whole
+  // 128-walker chunks; every split costs one FP64 atomic per output and plane.
+  const long want = (16L * 2 * 148 + n_jobs - 1) / n_jobs;
+  const int chunks = (W + 127) / 128;
+  const int splits = int(want < 1 ? 1 : want > chunks ? chunks : want);
+  const int per = (chunks + splits - 1) / splits * 128;
+  const dim3 grid(n_jobs, (W + per - 1) / per);
+  gram_simt_kernel<<<grid, kGramThreads, 0, st>>>(V, ldv, rec_w, ldw, W, per, jobs, out0, plane0,
+                                                  out1, plane1);
   return cudaPeekAtLastError() == cudaSuccess ? LEMC_OK : LEMC_ERR_CUDA;
 }
 

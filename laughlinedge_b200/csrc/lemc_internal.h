@@ -64,16 +64,20 @@ struct BasisProgram {
 // One tile of the SIMT FP64 Gram accumulation: three weighted sums
 //   out_h[a][b] += sum_w ONE(w) * P_h(w) * conj(v_a(w)) v_b(w),
 // P_h = rec_w plane plane[h] (plane[h] == LEMC_W_ONE: no extra factor,
-// plane[h] < 0: the sum is skipped).
+// plane[h] < 0: the sum is skipped).  The weights are real, so the transposed
+// block is the conjugate: mirror is its offset (-1: none to write), and only one
+// of two transposed tiles is a job.
 struct GramJob {
   int row_a;   // first V row of the Re part of sector a (Im rows follow at +Da)
   int Da;
   int row_b;
   int Db;
   int a0, b0;  // tile origin inside the (Da x Db) block
+  int ta, tb;  // tile shape, ta <= tb, each 8, 16 or 32
   int plane[3];
   int buf;     // 0: Gram planes, 1: cross planes
   int out;     // offset (in complex entries) of the (Da x Db) block in the output
+  int mirror;  // offset of the (Db x Da) block, or -1
 };
 
 int launch_sweep(const SweepArgs& a, int lanes_per_walker, cudaStream_t st);
@@ -104,8 +108,8 @@ int launch_learned_sweep(const SweepArgs& a, const void* wts, cudaStream_t st);
 int launch_advance_counters(uint32_t* ctr, cudaStream_t st);
 
 int launch_gram_simt(const float* V, int ldv, const float* rec_w, int ldw, int W,
-                     const GramJob* jobs, int n_jobs, int n_splits, double* out_set0,
-                     size_t plane0, double* out_set1, size_t plane1, cudaStream_t st);
+                     const GramJob* jobs, int n_jobs, double* out_set0, size_t plane0,
+                     double* out_set1, size_t plane1, cudaStream_t st);
 
 int launch_row_accumulate(const float* V, int ldv, const float* rec_w, int ldw, int W,
                           const int32_t* row_first, int n_rows, int D,
