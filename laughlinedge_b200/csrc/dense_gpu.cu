@@ -182,10 +182,9 @@ extern "C" int lemc_geneig_sweep(int D, const double* S, const double* H2, const
 // canonical orthogonalisation X of M (X^H M X = 1), C = X y and
 //   dy/dt = -i (H' + f(t) U') y,   H' = X^H H X - e I,  U' = X^H U X,
 // e = tr(H')/r removed as a global phase (no observable depends on it, and it
-// keeps h |H'| small).  Classical RK4 with h = save_step / substeps; every
-// stage is one fused kernel (axpy + the two matrix-vector products, one warp
-// per row).  Observables C^H rho_l C = y^H (X^H rho_l X) y and C^H M C = y^H y
-// are recorded on the device at every save point.
+// keeps h |H'| small).  Classical RK4 with h = save_step / substeps, up to
+// kObsBatch save points in one launch (rk4_kernel), then the observables
+// C^H rho_l C = y^H (X^H rho_l X) y and C^H M C = y^H y of the whole batch.
 namespace lemc {
 namespace {
 
@@ -223,73 +222,252 @@ __device__ __forceinline__ double2 cfma(double2 a, double2 b, double2 c) {
   return make_double2(fma(a.x, b.x, fma(-a.y, b.y, c.x)), fma(a.x, b.y, fma(a.y, b.x, c.y)));
 }
 
-// k_out = -i (H + f U) (y + a k_in), one warp per row; rows row-major.
-__global__ void rk_stage_kernel(int r, const double2* __restrict__ Hr, const double2* __restrict__ Ur,
-                                const double2* __restrict__ y, const double2* __restrict__ kin,
-                                double a, double f, double2* __restrict__ kout) {
-  const int row = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (row >= r) return;
-  double2 sh = make_double2(0.0, 0.0), su = make_double2(0.0, 0.0);
-  for (int j = lane; j < r; j += 32) {
-    double2 v = y[j];
-    if (kin) v = make_double2(fma(a, kin[j].x, v.x), fma(a, kin[j].y, v.y));
-    sh = cfma(Hr[size_t(row) * r + j], v, sh);
-    su = cfma(Ur[size_t(row) * r + j], v, su);
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    sh.x += __shfl_xor_sync(0xffffffffu, sh.x, o);
-    sh.y += __shfl_xor_sync(0xffffffffu, sh.y, o);
-    su.x += __shfl_xor_sync(0xffffffffu, su.x, o);
-    su.y += __shfl_xor_sync(0xffffffffu, su.y, o);
-  }
-  if (lane == 0) {
-    const double2 t = make_double2(sh.x + f * su.x, sh.y + f * su.y);
-    kout[row] = make_double2(t.y, -t.x);  // -i t
-  }
-}
+// Classical RK4 over many steps in one cooperative launch: k = -i (H + f U)(y + a k').
+//
+// A CTA owns `rpc` rows of H' and U' and keeps them in shared memory for the
+// whole launch (32 r^2 bytes over all CTAs: 60 KB each at r = 526; rows stay in
+// global memory, i.e. in L2, when they do not fit), with its own copy of y and
+// of the running RK sum, so a stage only exchanges the r entries of one k
+// vector through L2.  The stages are a serial chain of 4 grid barriers a step:
+// what bounds a step is their latency, not the r^2 work (8.8 MB of L2 reads or
+// 4.4 MFLOP a stage at r = 526).  Warps split a CTA's rows and columns.
+// One launch per stage and two warp-row products from L2 took 7.2 us a stage
+// plus the launch gaps; now 3.6 us a stage (526 states, 500 steps: 15.1 -> 7.1 ms).
+// Every grid barrier is bounded in time; on expiry the CTA raises *err and
+// leaves, and the others leave when they see it.
+constexpr int kObsBatch = 1024;  // save points per launch: bounds the Y buffer at 16 KB r
+constexpr int kRkThreads = 512;
+constexpr int kRkWarps = kRkThreads / 32;
+constexpr long long kRkWaitCycles = 4000000000LL;  // about 2 s
 
-__global__ void rk_update_kernel(int r, double h, double2* __restrict__ y, const double2* __restrict__ k1,
-                                 const double2* __restrict__ k2, const double2* __restrict__ k3,
-                                 const double2* __restrict__ k4) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= r) return;
-  const double c = h / 6.0;
-  y[i].x += c * (k1[i].x + 2.0 * k2[i].x + 2.0 * k3[i].x + k4[i].x);
-  y[i].y += c * (k1[i].y + 2.0 * k2[i].y + 2.0 * k3[i].y + k4[i].y);
-}
+struct RkArgs {
+  int r, rpc, parts;        // rows per CTA; warps per row (a power of two)
+  int rows_in_smem;
+  double2* ws;              // rows not in shared memory: 3 r entries a CTA for y, the sum, v
+  int v_in_smem;
+  const double2 *H, *U;     // row-major r x r
+  double2* y;               // state, in and out
+  double2* k;               // [2][r] exchange buffers
+  const double* f;          // profile at the three stage times of each step
+  double h;
+  int substeps, n_save;     // save points of this launch, substeps steps each
+  double2* Y;               // [n_save][r]: y at each save point
+  unsigned int* bar;        // arrivals so far
+  unsigned int bar0;        // arrivals before this launch
+  int* err;
+};
 
-// out[l] = y^H R_l y for the L row-major r x r matrices R, and nrm = y^H y;
-// one block per l (block L computes the norm).
-__global__ void observe_kernel(int r, int L, const double2* __restrict__ R, const double2* __restrict__ y,
-                               double2* __restrict__ out, double* __restrict__ nrm) {
-  __shared__ double2 red[256];
-  const int l = blockIdx.x;
-  double2 acc = make_double2(0.0, 0.0);
-  if (l < L) {
-    const double2* A = R + size_t(l) * r * r;
-    for (int i = threadIdx.x; i < r; i += blockDim.x) {
-      double2 row = make_double2(0.0, 0.0);
-      for (int j = 0; j < r; ++j) row = cfma(A[size_t(i) * r + j], y[j], row);
-      const double2 yc = make_double2(y[i].x, -y[i].y);
-      acc = cfma(yc, row, acc);
-    }
-  } else {
-    for (int i = threadIdx.x; i < r; i += blockDim.x) acc.x += y[i].x * y[i].x + y[i].y * y[i].y;
-  }
-  red[threadIdx.x] = acc;
+// All CTAs arrive; true when every arrival up to `target` is visible.
+__device__ __forceinline__ bool rk_barrier(const RkArgs& a, unsigned int target, int* ok) {
   __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) {
-      red[threadIdx.x].x += red[threadIdx.x + o].x;
-      red[threadIdx.x].y += red[threadIdx.x + o].y;
-    }
-    __syncthreads();
-  }
   if (threadIdx.x == 0) {
-    if (l < L) out[l] = red[0];
-    else *nrm = red[0].x;
+    __threadfence();
+    atomicAdd(a.bar, 1u);
+    const long long t0 = clock64();
+    int good = 1;
+    // counts are compared modulo 2^32
+    while (int(*(volatile unsigned int*)a.bar - target) < 0) {
+      if (*(volatile int*)a.err) { good = 0; break; }
+      if (clock64() - t0 > kRkWaitCycles) {
+        atomicExch(a.err, LEMC_ERR_TIMEOUT);
+        good = 0;
+        break;
+      }
+    }
+    __threadfence();
+    *ok = good;
   }
+  __syncthreads();
+  return *ok != 0;
+}
+
+__global__ void __launch_bounds__(kRkThreads, 1) rk4_kernel(const RkArgs a) {
+  extern __shared__ __align__(16) double2 rk_smem[];
+  __shared__ double2 part[kRkWarps];
+  __shared__ int ok;
+  const int r = a.r, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // y and the sum are read and written by one thread per entry; v is shared
+  double2* own = a.rows_in_smem ? rk_smem + r : a.ws + size_t(blockIdx.x) * 3 * r;
+  double2* y = own;                                     // [r]
+  double2* ks = own + r;                                // [r] k1 + 2 k2 + 2 k3
+  double2* v = a.v_in_smem ? rk_smem : own + 2 * r;     // [r] the stage's argument
+  double2* hs = rk_smem + 3 * r;                        // [rpc][r] (rows in shared memory)
+  double2* us = hs + size_t(a.rpc) * r;
+  const int row0 = blockIdx.x * a.rpc;
+  const int nrow = min(a.rpc, r - row0);
+  const double2* Hrow = a.H + size_t(row0) * r;
+  const double2* Urow = a.U + size_t(row0) * r;
+  if (a.rows_in_smem) {
+    for (int e = tid; e < nrow * r; e += kRkThreads) {
+      hs[e] = Hrow[e];
+      us[e] = Urow[e];
+    }
+    Hrow = hs;
+    Urow = us;
+  }
+  for (int j = tid; j < r; j += kRkThreads) y[j] = a.y[j];
+  __syncthreads();
+  const int rows_at_once = kRkWarps / a.parts;
+  unsigned int target = a.bar0;
+  size_t step = 0;
+  bool good = true;
+  for (int s = 0; s < a.n_save && good; ++s) {
+    for (int q = 0; q < a.substeps && good; ++q, ++step) {
+#pragma unroll 1
+      for (int st = 0; st < 4 && good; ++st) {
+        // argument of this stage from the previous stage's k
+        const double2* kin = a.k + size_t((st + 1) & 1) * r;
+        double2* kout = a.k + size_t(st & 1) * r;
+        const double c = st == 3 ? a.h : 0.5 * a.h;
+        if (st == 0) {
+          for (int j = tid; j < r; j += kRkThreads) v[j] = y[j];
+        } else {
+          for (int j = tid; j < r; j += kRkThreads) {
+            const double2 kj = __ldcg(kin + j);
+            const double2 yj = y[j];
+            v[j] = make_double2(fma(c, kj.x, yj.x), fma(c, kj.y, yj.y));
+            if (st == 1) {
+              ks[j] = kj;
+            } else {
+              ks[j].x += 2.0 * kj.x;
+              ks[j].y += 2.0 * kj.y;
+            }
+          }
+        }
+        __syncthreads();
+        const double f = a.f[3 * step + (st == 0 ? 0 : st == 3 ? 2 : 1)];
+        for (int b = 0; b < nrow; b += rows_at_once) {
+          const int row = b + warp / a.parts, p = warp % a.parts;
+          double2 sh = make_double2(0.0, 0.0), su = sh;
+          if (row < nrow) {
+            const double2* hr = Hrow + size_t(row) * r;
+            const double2* ur = Urow + size_t(row) * r;
+#pragma unroll 4
+            for (int j = p * 32 + lane; j < r; j += 32 * a.parts) {
+              const double2 x = v[j];
+              sh = cfma(hr[j], x, sh);
+              su = cfma(ur[j], x, su);
+            }
+          }
+          double2 t = make_double2(fma(f, su.x, sh.x), fma(f, su.y, sh.y));
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) {
+            t.x += __shfl_xor_sync(0xffffffffu, t.x, o);
+            t.y += __shfl_xor_sync(0xffffffffu, t.y, o);
+          }
+          if (lane == 0) part[warp] = t;
+          __syncthreads();
+          if (tid < rows_at_once && b + tid < nrow) {
+            double2 u = part[tid * a.parts];
+            for (int w = 1; w < a.parts; ++w) {
+              u.x += part[tid * a.parts + w].x;
+              u.y += part[tid * a.parts + w].y;
+            }
+            __stcg(kout + row0 + b + tid, make_double2(u.y, -u.x));  // -i u
+          }
+          __syncthreads();
+        }
+        target += gridDim.x;
+        good = rk_barrier(a, target, &ok);
+      }
+      if (!good) break;
+      const double c6 = a.h / 6.0;
+      const double2* k4 = a.k + size_t(1) * r;
+      for (int j = tid; j < r; j += kRkThreads) {
+        const double2 kj = __ldcg(k4 + j);
+        y[j].x += c6 * (ks[j].x + kj.x);
+        y[j].y += c6 * (ks[j].y + kj.y);
+      }
+      __syncthreads();
+    }
+    if (good)
+      for (int j = row0 + tid; j < row0 + nrow; j += kRkThreads) a.Y[size_t(s) * r + j] = y[j];
+  }
+  if (good)
+    for (int j = row0 + tid; j < row0 + nrow; j += kRkThreads) a.y[j] = y[j];
+}
+
+// out[z][s][l] = sum over row tiles x = z, z + Z, ... of y_s^H R_l y_s, for a
+// batch of save points (rows of Y) at once; l == L gives y^H y.  A block takes 32
+// save points of one l: R_l Y^T in 32 x 32 tiles (2 x 2 entries a thread, operands
+// staged in shared memory), each multiplied by conj(y) as it is done.  4 FP64 FMAs
+// per entry, so the FP64 pipe bounds it; one thread per matrix row and save point
+// (uncoalesced rows, L + 1 blocks) took 191 us a save point
+// (526 states, 9 components; now 1.3 us).
+constexpr int kObsT = 32, kObsThreads = 256, kObsZ = 4;
+
+__global__ void __launch_bounds__(kObsThreads)
+observe_kernel(int r, int L, const double2* __restrict__ R, const double2* __restrict__ Y, int n,
+               double2* __restrict__ out) {
+  __shared__ double2 ra[kObsT][kObsT + 1], ys[kObsT][kObsT + 1];  // [j][row], [j][save]
+  const int s0 = blockIdx.x * kObsT, l = blockIdx.y, z = blockIdx.z;
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const double2 zero = make_double2(0.0, 0.0);
+  double2 acc[2] = {zero, zero};  // save points s0 + tx, s0 + tx + 16
+  const double2* A = R + size_t(l < L ? l : 0) * r * r;
+  for (int i0 = z * kObsT; i0 < r; i0 += kObsZ * kObsT) {
+    double2 t[2][2] = {{zero, zero}, {zero, zero}};  // [row][save]
+    if (l < L) {
+      for (int j0 = 0; j0 < r; j0 += kObsT) {
+        __syncthreads();
+        for (int e = tid; e < kObsT * kObsT; e += kObsThreads) {
+          const int j = e & 31, q = e >> 5;
+          ra[j][q] = (i0 + q < r && j0 + j < r) ? A[size_t(i0 + q) * r + j0 + j] : zero;
+          ys[j][q] = (s0 + q < n && j0 + j < r) ? Y[size_t(s0 + q) * r + j0 + j] : zero;
+        }
+        __syncthreads();
+#pragma unroll 8
+        for (int j = 0; j < kObsT; ++j) {
+          const double2 a0 = ra[j][ty], a1 = ra[j][ty + 16];
+          const double2 b0 = ys[j][tx], b1 = ys[j][tx + 16];
+          t[0][0] = cfma(a0, b0, t[0][0]);
+          t[0][1] = cfma(a0, b1, t[0][1]);
+          t[1][0] = cfma(a1, b0, t[1][0]);
+          t[1][1] = cfma(a1, b1, t[1][1]);
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int row = i0 + ty + 16 * i, s = s0 + tx + 16 * q;
+        if (row >= r || s >= n) continue;
+        const double2 y = Y[size_t(s) * r + row];
+        const double2 m = l < L ? t[i][q] : y;
+        acc[q] = cfma(make_double2(y.x, -y.y), m, acc[q]);
+      }
+  }
+  __syncthreads();
+  ra[ty][tx] = acc[0];
+  ra[ty][tx + 16] = acc[1];
+  __syncthreads();
+  if (tid < kObsT && s0 + tid < n) {
+    double2 v = ra[0][tid];
+    for (int q = 1; q < 16; ++q) {
+      v.x += ra[q][tid].x;
+      v.y += ra[q][tid].y;
+    }
+    out[(size_t(z) * n + s0 + tid) * (L + 1) + l] = v;
+  }
+}
+
+// sums of the kObsZ partial observables of a batch: obs[n][L] and nrm[n]
+__global__ void observe_sum_kernel(int n, int L, const double2* __restrict__ part,
+                                   double2* __restrict__ obs, double* __restrict__ nrm) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= n * (L + 1)) return;
+  double2 v = part[e];
+  for (int z = 1; z < kObsZ; ++z) {
+    const double2 p = part[size_t(z) * n * (L + 1) + e];
+    v.x += p.x;
+    v.y += p.y;
+  }
+  const int s = e / (L + 1), l = e % (L + 1);
+  if (l < L)
+    obs[size_t(s) * L + l] = v;
+  else
+    nrm[s] = v.x;
 }
 
 }  // namespace
@@ -361,11 +539,18 @@ extern "C" int lemc_evolve_device(int D, const double* M, const double* H, const
   double2* Rr = g.alloc<double2>(RR * std::max(1, L));
   double2* A = g.alloc<double2>(RR);
   double* emean = g.alloc<double>(1);
-  double2 *y = g.alloc<double2>(r), *k1 = g.alloc<double2>(r), *k2 = g.alloc<double2>(r),
-          *k3 = g.alloc<double2>(r), *k4 = g.alloc<double2>(r);
+  const int batch = std::min(ns, kObsBatch);
+  const double h = save_step / substeps;
+  const size_t nsteps = size_t(ns > 1 ? ns - 1 : 0) * substeps;
+  double2 *y = g.alloc<double2>(r), *kx = g.alloc<double2>(2 * size_t(r));
+  double2* Y = g.alloc<double2>(size_t(batch) * r);
+  double2* obs_part = g.alloc<double2>(size_t(kObsZ) * batch * (L + 1));
   double2* obs = g.alloc<double2>(size_t(ns) * std::max(1, L));
   double* nrm = g.alloc<double>(ns);
-  if (!Hr || !Ur || !Rr || !A || !emean || !y || !k1 || !k2 || !k3 || !k4 || !obs || !nrm)
+  double* dfv = g.alloc<double>(std::max<size_t>(1, 3 * nsteps));
+  int* sync = g.alloc<int>(2);  // barrier arrivals, error word
+  if (!Hr || !Ur || !Rr || !A || !emean || !y || !kx || !Y || !obs_part || !obs || !nrm || !dfv ||
+      !sync)
     return LEMC_ERR_CUDA;
   const cuDoubleComplex one = make_cuDoubleComplex(1.0, 0.0), zero = make_cuDoubleComplex(0.0, 0.0);
   auto project = [&](const double2* Bcm) -> bool {  // A = X^H B X (column-major r x r)
@@ -397,8 +582,6 @@ extern "C" int lemc_evolve_device(int D, const double* M, const double* H, const
     return LEMC_ERR_CUDA;
   if (cudaPeekAtLastError() != cudaSuccess) return LEMC_ERR_CUDA;
   // profile values at every stage time, evaluated on the host
-  const double h = save_step / substeps;
-  const size_t nsteps = size_t(ns > 1 ? ns - 1 : 0) * substeps;
   std::vector<double> fv(3 * nsteps);
   for (size_t k = 0; k < nsteps; ++k) {
     const double t = double(k) * h;
@@ -406,21 +589,70 @@ extern "C" int lemc_evolve_device(int D, const double* M, const double* H, const
     fv[3 * k + 1] = f ? f(t + 0.5 * h, user) : 0.0;
     fv[3 * k + 2] = f ? f(t + h, user) : 0.0;
   }
-  const int wpb = 8, sblocks = (r + wpb - 1) / wpb, ublocks = (r + 255) / 256;
-  observe_kernel<<<L + 1, 256>>>(r, L, Rr, y, obs, nrm);
-  size_t k = 0;
-  for (int s = 1; s < ns; ++s) {
-    for (int q = 0; q < substeps; ++q, ++k) {
-      rk_stage_kernel<<<sblocks, 32 * wpb>>>(r, Hr, Ur, y, nullptr, 0.0, fv[3 * k], k1);
-      rk_stage_kernel<<<sblocks, 32 * wpb>>>(r, Hr, Ur, y, k1, 0.5 * h, fv[3 * k + 1], k2);
-      rk_stage_kernel<<<sblocks, 32 * wpb>>>(r, Hr, Ur, y, k2, 0.5 * h, fv[3 * k + 1], k3);
-      rk_stage_kernel<<<sblocks, 32 * wpb>>>(r, Hr, Ur, y, k3, h, fv[3 * k + 2], k4);
-      rk_update_kernel<<<ublocks, 256>>>(r, h, y, k1, k2, k3, k4);
+  if (nsteps > 0 && cudaMemcpy(dfv, fv.data(), sizeof(double) * fv.size(), cudaMemcpyHostToDevice) != cudaSuccess)
+    return LEMC_ERR_CUDA;
+  if (cudaMemset(sync, 0, 2 * sizeof(int)) != cudaSuccess) return LEMC_ERR_CUDA;
+  // One CTA per SM at most, at least four rows each (a barrier costs more with
+  // more CTAs than fewer rows save); rows in shared memory when they fit.
+  int dev = 0, sms = 148, smem_max = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
+    return LEMC_ERR_CUDA;
+  RkArgs ra{};
+  ra.r = r;
+  ra.rpc = std::max(4, (r + sms - 1) / sms);
+  ra.parts = kRkWarps;
+  while (ra.parts > 1 && kRkWarps / ra.parts < ra.rpc) ra.parts /= 2;
+  const size_t vec_bytes = sizeof(double2) * size_t(r);
+  const size_t row_bytes = 2 * vec_bytes * size_t(ra.rpc);
+  const size_t smem_cap = size_t(smem_max) - 1024;  // the kernel's static shared memory
+  ra.rows_in_smem = 3 * vec_bytes + row_bytes <= smem_cap;
+  ra.v_in_smem = vec_bytes <= smem_cap;
+  const size_t rk_smem_bytes = ra.rows_in_smem ? 3 * vec_bytes + row_bytes : ra.v_in_smem ? vec_bytes : 0;
+  if (cudaFuncSetAttribute(rk4_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           int(rk_smem_bytes)) != cudaSuccess)
+    return LEMC_ERR_CUDA;
+  const int rk_ctas = (r + ra.rpc - 1) / ra.rpc;
+  if (!ra.rows_in_smem) {
+    ra.ws = g.alloc<double2>(size_t(rk_ctas) * 3 * r);
+    if (!ra.ws) return LEMC_ERR_CUDA;
+  }
+  ra.H = Hr;
+  ra.U = Ur;
+  ra.y = y;
+  ra.k = kx;
+  ra.h = h;
+  ra.substeps = substeps;
+  ra.bar = reinterpret_cast<unsigned int*>(sync);
+  ra.err = sync + 1;
+  // save point 0 is the initial state; the others follow in batches
+  if (cudaMemcpyAsync(Y, y, sizeof(double2) * r, cudaMemcpyDeviceToDevice) != cudaSuccess)
+    return LEMC_ERR_CUDA;
+  for (int s0 = 0, first = 1; s0 < ns; first = 0) {
+    const int n = std::min(batch, ns - s0);
+    ra.n_save = n - first;
+    ra.Y = Y + size_t(first) * r;
+    ra.f = dfv + 3 * size_t(s0 + first - 1) * substeps;
+    if (ra.n_save > 0) {
+      void* kargs[] = {&ra};
+      if (cudaLaunchCooperativeKernel(reinterpret_cast<void*>(rk4_kernel), dim3(rk_ctas),
+                                      dim3(kRkThreads), kargs, rk_smem_bytes, nullptr) != cudaSuccess)
+        return LEMC_ERR_CUDA;
+      ra.bar0 += 4u * unsigned(ra.n_save) * unsigned(substeps) * unsigned(rk_ctas);
     }
-    observe_kernel<<<L + 1, 256>>>(r, L, Rr, y, obs + size_t(s) * std::max(1, L), nrm + s);
+    observe_kernel<<<dim3((n + kObsT - 1) / kObsT, L + 1, kObsZ), kObsThreads>>>(r, L, Rr, Y, n,
+                                                                                obs_part);
+    observe_sum_kernel<<<(n * (L + 1) + 255) / 256, 256>>>(n, L, obs_part, obs + size_t(s0) * L,
+                                                          nrm + s0);
+    s0 += n;
   }
   if (cudaPeekAtLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess)
     return LEMC_ERR_CUDA;
+  int rk_err = 0;
+  if (cudaMemcpy(&rk_err, ra.err, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess)
+    return LEMC_ERR_CUDA;
+  if (rk_err != 0) return LEMC_ERR_TIMEOUT;
   if (L > 0 && out) {
     std::vector<double2> all(size_t(ns) * L);
     if (cudaMemcpy(all.data(), obs, all.size() * sizeof(double2), cudaMemcpyDeviceToHost) != cudaSuccess)
