@@ -57,7 +57,8 @@ enum lemc_gram_mode {
   LEMC_GRAM_FP64 = 0,   /* SIMT FP64 accumulation (the exact accumulation)     */
   LEMC_GRAM_BF16X3 = 1, /* tcgen05 kind::f16, hi/lo split, 3 products         */
   LEMC_GRAM_BF16X4 = 2, /* tcgen05 kind::f16, hi/lo split, 4 products         */
-  LEMC_GRAM_TF32X3 = 3  /* tcgen05 kind::tf32, hi/lo split, 3 products        */
+  LEMC_GRAM_TF32X3 = 3  /* tcgen05, 22-bit hi/lo split (two row-scaled FP16
+                           terms, as precise as two TF32 terms), 3 products   */
 };
 /* weight planes recorded per measurement (rows of the record buffer) */
 enum lemc_weight {

@@ -83,7 +83,7 @@ template <int P>
 __global__ void __launch_bounds__(kBasisThreads)
 basis_kernel(const float2* __restrict__ rec_p, int W, int K, float pN, BasisProgram prog,
              float* __restrict__ V, int ldv, double* __restrict__ series,
-             const uint32_t* __restrict__ series_idx) {
+             const uint32_t* __restrict__ series_idx, const RangeOut rng) {
   // Shared memory, one column of P values per thread (no thread reads
   // another's column):
   //   ps[k][thread]  = p_k of the thread's walkers, k = 0..K (p_0 = N)
@@ -145,6 +145,32 @@ basis_kernel(const float2* __restrict__ rec_p, int W, int K, float pN, BasisProg
       atomicAdd(&series[tid], v);
     }
   }
+  if (rng.range && blockIdx.y == 0) {
+    // largest |p_k|^2 and weight magnitudes over the walkers, as FP32 bits
+    for (int k = 1; k <= K; ++k) {
+      const Vals<P> pk = vload<P>(ps + k * R);
+      uint32_t m = 0u;
+#pragma unroll
+      for (int i = 0; i < P; ++i)
+        m = max(m, __float_as_uint(fmaf(pk.c[i].x, pk.c[i].x, pk.c[i].y * pk.c[i].y)));
+      m = __reduce_max_sync(0xffffffffu, m);
+      if ((tid & 31) == 0) atomicMax(rng.p2max + k, m);
+    }
+    uint32_t m[3] = {0u, 0u, 0u};
+    for (int i = 0; live && i < P; ++i) {
+      const float w1 = rng.rec_w[w0 + i];
+#pragma unroll
+      for (int h = 0; h < 3; ++h) {
+        const float v = h == 0 ? w1 : w1 * rng.rec_w[size_t(h) * rng.ldw + w0 + i];
+        m[h] = max(m[h], __float_as_uint(v) & 0x7FFFFFFFu);
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < 3; ++h) {
+      const uint32_t v = __reduce_max_sync(0xffffffffu, m[h]);
+      if ((tid & 31) == 0) atomicMax(rng.range + rng.rows + h, v);
+    }
+  }
   __syncthreads();  // the program segment is in shared memory
   if (!live) return;
 
@@ -193,9 +219,38 @@ basis_kernel(const float2* __restrict__ rec_p, int W, int K, float pN, BasisProg
   }
 }
 
+// Bound on max |v_a| = c_a prod_k |p_k|^{r_k} over the walkers from the largest
+// |p_k|, as a power of two (its FP32 bits), for both V rows of state a.  The 0.01
+// covers the FP32 rounding of the products and of these logarithms.  The bound
+// exceeds the maximum by the product of maxima not met by one walker (2^4 to 2^12
+// for droplets at up to 131072 walkers), which the split's 2^40 between the top of
+// FP16's range and its smallest term absorbs.  Maxima of V itself cost a third of
+// the basis build inside it (0.30 -> 0.49 ms at 2713 states and 65536 walkers), or
+// another read of V (0.21 ms); this costs 3 us.
+__global__ void row_bound_kernel(const RangeOut rng) {
+  const int a = blockIdx.x * blockDim.x + threadIdx.x;
+  if (a >= rng.states) return;
+  float lb = log2f(rng.row_scale[a]);
+  bool finite = true, zero = false;
+  for (int k = 1; k < rng.ldm; ++k) {
+    const int r = rng.mult[a * rng.ldm + k];
+    if (r == 0) continue;
+    const float p2 = __uint_as_float(rng.p2max[k]);
+    finite = finite && p2 <= 3.0e38f;
+    zero = zero || p2 == 0.f;
+    lb += 0.5f * float(r) * log2f(p2);
+  }
+  if (rng.mult[a * rng.ldm]) lb += log2f(rng.p0);
+  const int e = int(floorf(fminf(fmaxf(lb + 0.01f, -127.f), 128.f)));
+  const uint32_t bits = !finite ? 0x7F800000u : zero ? 0u : uint32_t(e + 127) << 23;
+  rng.range[rng.row_re[a]] = bits;
+  rng.range[rng.row_im[a]] = bits;
+}
+
 template <int P>
 int launch_p(const float2* rec_p, int W, int K, int N, const BasisProgram& prog, float* V,
-             int ldv, double* series, const uint32_t* series_idx, cudaStream_t st) {
+             int ldv, double* series, const uint32_t* series_idx, const RangeOut& rng,
+             cudaStream_t st) {
   const size_t smem = sizeof(float2) * size_t(2 * K + 1) * kBasisThreads * P +
                       (sizeof(BasisNode) + sizeof(float)) * size_t(prog.max_seg + 2);
   if (smem > 40 * 1024) {  // the static reduction buffer shares the 48 KiB default
@@ -208,7 +263,7 @@ int launch_p(const float2* rec_p, int W, int K, int N, const BasisProgram& prog,
   const int per_block = kBasisThreads * P;
   const dim3 grid((W + per_block - 1) / per_block, prog.n_seg);
   basis_kernel<P><<<grid, kBasisThreads, smem, st>>>(rec_p, W, K, float(N), prog, V, ldv,
-                                                     series, series_idx);
+                                                     series, series_idx, rng);
   return cudaPeekAtLastError() == cudaSuccess ? LEMC_OK : LEMC_ERR_CUDA;
 }
 
@@ -230,7 +285,8 @@ int launch_multipole_plane(const float2* rec_p, int W, int K, int k, double scal
 }
 
 int launch_basis(const float2* rec_p, int W, int K, int N, const BasisProgram& prog, float* V,
-                 int ldv, double* series, const uint32_t* series_idx, cudaStream_t st) {
+                 int ldv, double* series, const uint32_t* series_idx, const RangeOut& rng,
+                 cudaStream_t st) {
   if (K > kMaxDegree || prog.max_part > K || prog.max_depth > K || prog.n_seg < 1 ||
       prog.n_seg > kMaxBasisSegments)
     return LEMC_ERR_CAPACITY;
@@ -239,8 +295,15 @@ int launch_basis(const float2* rec_p, int W, int K, int N, const BasisProgram& p
   const bool pairs = W % 2 == 0 && ldv % 2 == 0 &&
                      reinterpret_cast<uintptr_t>(rec_p) % 16 == 0 &&
                      reinterpret_cast<uintptr_t>(V) % 8 == 0;
-  return pairs ? launch_p<2>(rec_p, W, K, N, prog, V, ldv, series, series_idx, st)
-               : launch_p<1>(rec_p, W, K, N, prog, V, ldv, series, series_idx, st);
+  // the weights' and the |p_k|^2 maxima are neighbours behind the row bounds
+  if (rng.range && cudaMemsetAsync(rng.range + rng.rows, 0, sizeof(uint32_t) * (3 + kMaxDegree + 1),
+                                   st) != cudaSuccess)
+    return LEMC_ERR_CUDA;
+  const int s = pairs ? launch_p<2>(rec_p, W, K, N, prog, V, ldv, series, series_idx, rng, st)
+                      : launch_p<1>(rec_p, W, K, N, prog, V, ldv, series, series_idx, rng, st);
+  if (s != LEMC_OK || !rng.range) return s;
+  row_bound_kernel<<<(rng.states + 127) / 128, 128, 0, st>>>(rng);
+  return cudaPeekAtLastError() == cudaSuccess ? LEMC_OK : LEMC_ERR_CUDA;
 }
 
 }  // namespace lemc

@@ -180,6 +180,8 @@ struct lemc_ctx {
   std::vector<double> row_scale;      // per basis row
   std::vector<BasisNode> prog_host;   // the basis program (with its sentinels)
   DevBuf<float> d_node_scale;         // per program node
+  DevBuf<float> d_row_scale;          // per basis row
+  DevBuf<uint8_t> d_row_mult;         // [D][K + 1] multiplicities of the parts 0..K
   bool scale_pending = false;
   bool gram_tune_pending = false;  // autotune the contraction's walker split
   int gram_splits = 0;             // the tuned split (0: one-wave rule)
@@ -208,8 +210,11 @@ struct lemc_ctx {
   // tcgen05 path
   std::vector<TcTile> tc_tiles;
   int tc_ntiles = 0, tc_maxdim = 0;
+  int tc_njobs = 0, tc_panels = 1;  // contraction jobs; B panels (tiles) per job
   DevBuf<TcSector> d_tc_secs;
-  DevBuf<TcTile> d_tc_tiles;
+  DevBuf<TcTile> d_tc_tiles;  // every tile of every split (first n_tiles: split 0)
+  DevBuf<TcTile> d_tc_jobs;   // the contraction's jobs
+  DevBuf<uint32_t> d_tc_range;  // largest magnitude of each V row and weight plane
   DevBuf<double> tc_partials;
   int tc_splits = 1;
 
@@ -468,10 +473,6 @@ int upload_guide(lemc_ctx* c) {
   LEMC_TRY(c->d_row_first.alloc(R + 1));
   LEMC_CUDA(cudaMemcpy(c->d_walker_row.p, c->walker_row.data(), 4 * c->W, cudaMemcpyHostToDevice));
   LEMC_CUDA(cudaMemcpy(c->d_row_first.p, c->row_first.data(), 4 * (R + 1), cudaMemcpyHostToDevice));
-  LEMC_TRY(c->d_row_re.alloc(R));
-  LEMC_TRY(c->d_row_im.alloc(R));
-  LEMC_CUDA(cudaMemcpy(c->d_row_re.p, c->row_vre.data(), 4 * R, cudaMemcpyHostToDevice));
-  LEMC_CUDA(cudaMemcpy(c->d_row_im.p, c->row_vim.data(), 4 * R, cudaMemcpyHostToDevice));
   LEMC_TRY(c->rowacc.alloc(size_t(R) * R * kRowAcc));
   LEMC_CUDA(cudaMemset(c->rowacc.p, 0, sizeof(double) * R * R * kRowAcc));
   return LEMC_OK;
@@ -516,7 +517,31 @@ int sweep_once(lemc_ctx* c, int n_sweeps, int measure) {
   return launch_sweep_for(c, sweep_args(c, n_sweeps, measure));
 }
 
-int gram_step(lemc_ctx* c, const float* V, const float* rec_w, int ldw, int W, int mode) {
+// The basis build of the context's own V also records the operand ranges that a
+// tensor-core contraction of it will need.
+int basis_step(lemc_ctx* c, double* series, const uint32_t* series_idx) {
+  RangeOut rng;
+  if (c->cfg.guide != LEMC_GUIDE_ROW && c->cfg.gram_mode != LEMC_GRAM_FP64) {
+    if (c->tc_tiles.empty()) LEMC_TRY(setup_tc(c, c->gram_splits));
+    rng.range = c->d_tc_range.p;
+    rng.rows = 2 * c->D;
+    rng.rec_w = c->rec_w.p;
+    rng.ldw = c->Wpad;
+    rng.p2max = rng.range + rng.rows + 3;
+    rng.states = c->D;
+    rng.mult = c->d_row_mult.p;
+    rng.ldm = c->K + 1;
+    rng.row_scale = c->d_row_scale.p;
+    rng.row_re = c->d_row_re.p;
+    rng.row_im = c->d_row_im.p;
+    rng.p0 = float(c->N);
+  }
+  return launch_basis(c->rec_p.p, c->W, c->K, c->N, c->bprog, c->V.p, c->Wpad, series, series_idx,
+                      rng, c->stream);
+}
+
+// own_v: V is the context's, just written by basis_step (its ranges are known)
+int gram_step(lemc_ctx* c, const float* V, const float* rec_w, int ldw, int W, int mode, bool own_v) {
   if (c->cfg.guide == LEMC_GUIDE_ROW) {
     return launch_row_accumulate(V, c->Wpad, rec_w, ldw, W, c->d_row_first.p,
                                  int(c->basis.rows.size()), c->D, c->d_row_re.p, c->d_row_im.p,
@@ -530,9 +555,9 @@ int gram_step(lemc_ctx* c, const float* V, const float* rec_w, int ldw, int W, i
                             c->gram_plane, c->cross.p, c->cross_plane, c->stream);
   }
   if (c->tc_tiles.empty()) LEMC_TRY(setup_tc(c, c->gram_splits));
-  int s = launch_gram_tc_rows(V, c->Wpad, 2 * c->D, rec_w, ldw, c->Wpad, c->d_tc_tiles.p,
-                              int(c->tc_tiles.size()), c->tc_splits, c->tc_partials.p, mode,
-                              c->cfg.flush_every, c->err.p, c->stream);
+  int s = launch_gram_tc_rows(V, c->Wpad, 2 * c->D, rec_w, ldw, c->Wpad, c->d_tc_jobs.p,
+                              c->tc_njobs, c->tc_panels, c->tc_splits, c->d_tc_range.p,
+                              own_v, c->tc_partials.p, mode, c->cfg.flush_every, c->err.p, c->stream);
   if (s != LEMC_OK) return s;
   // cross-sector planes (user potential, cos/sin probes): FP64 path
   if (cross) {
@@ -618,12 +643,32 @@ int setup_tc(lemc_ctx* c, int force_splits) {
   c->tc_tiles.clear();
   for (int sp = 0; sp < c->tc_splits; ++sp)
     for (int t = 0; t < nt; ++t)
-      c->tc_tiles.push_back({tiles[t].first, tiles[t].second, sp, sp * nt + t});
+      c->tc_tiles.push_back({tiles[t].first, tiles[t].second, sp, sp * nt + t, 1});
+  // Jobs: two neighbouring tiles of one A slice together when that still leaves a
+  // job for every SM, else one tile each: a pair converts and loads its A operand
+  // once (2713 states 3.0 against 4.0 ms, 526 states 0.39 against 0.45 ms), but 272
+  // states have 77 pairs for 148 SMs and take 0.20 against 0.16 ms.
+  std::vector<TcTile> jobs;
+  for (size_t t = 0; t < c->tc_tiles.size(); ++t) {
+    TcTile jb = c->tc_tiles[t];
+    if (t + 1 < c->tc_tiles.size() && c->tc_tiles[t + 1].ksplit == jb.ksplit &&
+        c->tc_tiles[t + 1].row0 == jb.row0 && c->tc_tiles[t + 1].col0 == jb.col0 + 32) {
+      jb.panels = 2;
+      ++t;
+    }
+    jobs.push_back(jb);
+  }
+  c->tc_panels = int(jobs.size()) >= sm ? 2 : 1;
+  if (c->tc_panels == 1) jobs = c->tc_tiles;
+  c->tc_njobs = int(jobs.size());
+  LEMC_TRY(c->d_tc_jobs.alloc(jobs.size()));
+  LEMC_CUDA(cudaMemcpy(c->d_tc_jobs.p, jobs.data(), sizeof(TcTile) * jobs.size(), cudaMemcpyHostToDevice));
   LEMC_TRY(c->d_tc_tiles.alloc(c->tc_tiles.size()));
   LEMC_CUDA(cudaMemcpy(c->d_tc_tiles.p, c->tc_tiles.data(), sizeof(TcTile) * c->tc_tiles.size(),
                        cudaMemcpyHostToDevice));
   LEMC_TRY(c->d_tc_secs.alloc(ns));
   LEMC_CUDA(cudaMemcpy(c->d_tc_secs.p, secs.data(), sizeof(TcSector) * ns, cudaMemcpyHostToDevice));
+  LEMC_TRY(c->d_tc_range.alloc(2 * size_t(c->D) + 3 + kMaxDegree + 1));
   const size_t slot = size_t(kTcSlot);
   LEMC_TRY(c->tc_partials.alloc(slot * c->tc_tiles.size()));
   LEMC_CUDA(cudaMemsetAsync(c->tc_partials.p, 0, sizeof(double) * slot * c->tc_tiles.size(),
@@ -773,9 +818,13 @@ int lemc_destroy(lemc_ctx* c) {
   c->rowacc.release();
   c->err.release();
   c->d_tc_tiles.release();
+  c->d_tc_jobs.release();
   c->d_tc_secs.release();
   c->tc_partials.release();
+  c->d_tc_range.release();
   c->d_node_scale.release();
+  c->d_row_scale.release();
+  c->d_row_mult.release();
   for (auto& e : c->ev)
     if (e) cudaEventDestroy(e);
   for (auto& e : c->pev) cudaEventDestroy(e);
@@ -829,6 +878,20 @@ int lemc_set_sectors(lemc_ctx* c, const int32_t* sectors, int n) {
                          cudaMemcpyHostToDevice));
   }
   c->bprog.node_scale = c->d_node_scale.p;
+  {
+    std::vector<uint8_t> mult(size_t(c->D) * (c->K + 1), 0);
+    for (int r = 0; r < c->D; ++r)
+      for (const auto& pp : c->basis.rows[r].pairs) mult[size_t(r) * (c->K + 1) + pp.part] = uint8_t(pp.mult);
+    const std::vector<float> ones(c->D, 1.f);
+    LEMC_TRY(c->d_row_mult.alloc(mult.size()));
+    LEMC_TRY(c->d_row_scale.alloc(c->D));
+    LEMC_TRY(c->d_row_re.alloc(c->D));
+    LEMC_TRY(c->d_row_im.alloc(c->D));
+    LEMC_CUDA(cudaMemcpy(c->d_row_mult.p, mult.data(), mult.size(), cudaMemcpyHostToDevice));
+    LEMC_CUDA(cudaMemcpy(c->d_row_scale.p, ones.data(), 4 * ones.size(), cudaMemcpyHostToDevice));
+    LEMC_CUDA(cudaMemcpy(c->d_row_re.p, c->row_vre.data(), 4 * c->D, cudaMemcpyHostToDevice));
+    LEMC_CUDA(cudaMemcpy(c->d_row_im.p, c->row_vim.data(), 4 * c->D, cudaMemcpyHostToDevice));
+  }
   c->scale_pending = c->cfg.guide == LEMC_GUIDE_LAUGHLIN;
   c->gram_tune_pending = c->cfg.lanes_per_walker < 0 && c->cfg.guide == LEMC_GUIDE_LAUGHLIN &&
                          c->cfg.gram_mode != LEMC_GRAM_FP64;
@@ -1031,10 +1094,9 @@ static int graph_step(lemc_ctx* c) {
   a.sweep0 = 0;
   a.sweep_ctr = c->d_ctr.p;
   LEMC_TRY(launch_sweep_for(c, a));
-  LEMC_TRY(launch_basis(c->rec_p.p, c->W, c->K, c->N, c->bprog, c->V.p, c->Wpad,
-                        c->series.p, c->d_ctr.p + 1, c->stream));
+  LEMC_TRY(basis_step(c, c->series.p, c->d_ctr.p + 1));
   LEMC_TRY(multipole_step(c));
-  LEMC_TRY(gram_step(c, c->V.p, c->rec_w.p, c->Wpad, c->W, c->cfg.gram_mode));
+  LEMC_TRY(gram_step(c, c->V.p, c->rec_w.p, c->Wpad, c->W, c->cfg.gram_mode, true));
   return launch_advance_counters(c->d_ctr.p, c->stream);
 }
 
@@ -1117,6 +1179,10 @@ static int compute_row_scales(lemc_ctx* c) {
     vrow[c->row_vre[r]] = scf;
     vrow[c->row_vim[r]] = scf;
   }
+  std::vector<float> rows(D);
+  for (int r = 0; r < D; ++r) rows[r] = float(c->row_scale[r]);
+  LEMC_CUDA(cudaMemcpyAsync(c->d_row_scale.p, rows.data(), sizeof(float) * rows.size(),
+                            cudaMemcpyHostToDevice, c->stream));
   std::vector<float> dev(c->prog_host.size(), 1.f);  // per program node
   for (size_t t = 0; t < dev.size(); ++t)
     if (c->prog_host[t].row_re >= 0) dev[t] = vrow[c->prog_host[t].row_re];
@@ -1151,16 +1217,16 @@ static int autotune_gram_splits(lemc_ctx* c) {
   LEMC_CUDA(cudaMemcpyAsync(save.p, c->pos.p, sizeof(float2) * c->W * c->N,
                             cudaMemcpyDeviceToDevice, c->stream));
   LEMC_TRY(sweep_once(c, 1, 1));
-  LEMC_TRY(launch_basis(c->rec_p.p, c->W, c->K, c->N, c->bprog, c->V.p, c->Wpad, nullptr,
-                        nullptr, c->stream));
+  LEMC_TRY(basis_step(c, nullptr, nullptr));
   float best = 1e30f;
   int best_sp = cand[0];
   for (int sp : cand) {
     LEMC_TRY(setup_tc(c, sp));
     auto launch = [&]() {
       return launch_gram_tc_rows(c->V.p, c->Wpad, 2 * c->D, c->rec_w.p, c->Wpad, c->Wpad,
-                                 c->d_tc_tiles.p, int(c->tc_tiles.size()), c->tc_splits,
-                                 c->tc_partials.p, c->cfg.gram_mode, c->cfg.flush_every, c->err.p,
+                                 c->d_tc_jobs.p, c->tc_njobs, c->tc_panels, c->tc_splits,
+                                 c->d_tc_range.p, true, c->tc_partials.p, c->cfg.gram_mode,
+                                 c->cfg.flush_every, c->err.p,
                                  c->stream);
     };
     LEMC_TRY(launch());  // warm
@@ -1243,8 +1309,7 @@ static int run_impl(lemc_ctx* c, int n_sweeps, int measure, lemc_step_hook hook,
     LEMC_TRY(sweep_once(c, 1, 1));
     c->sweeps += 1;
     if (c->profile) LEMC_CUDA(cudaEventRecord(c->pev[4 * s + 1], c->stream));
-    LEMC_TRY(launch_basis(c->rec_p.p, c->W, c->K, c->N, c->bprog, c->V.p, c->Wpad,
-                          c->series.p + 8 * size_t(s), nullptr, c->stream));
+    LEMC_TRY(basis_step(c, c->series.p + 8 * size_t(s), nullptr));
     LEMC_TRY(multipole_step(c));
     if (hook) {
       if (!c->hooked) ++c->version;
@@ -1255,7 +1320,7 @@ static int run_impl(lemc_ctx* c, int n_sweeps, int measure, lemc_step_hook hook,
       if (hs != LEMC_OK) return hs;
     }
     if (c->profile) LEMC_CUDA(cudaEventRecord(c->pev[4 * s + 2], c->stream));
-    LEMC_TRY(gram_step(c, c->V.p, c->rec_w.p, c->Wpad, c->W, c->cfg.gram_mode));
+    LEMC_TRY(gram_step(c, c->V.p, c->rec_w.p, c->Wpad, c->W, c->cfg.gram_mode, true));
     if (c->profile) LEMC_CUDA(cudaEventRecord(c->pev[4 * s + 3], c->stream));
     c->meas += 1;
   }
@@ -1490,7 +1555,7 @@ int lemc_basis_device(lemc_ctx* c, const void* rec_p, int W, void* V, int ldv, v
   if (!c->has_basis) return LEMC_ERR_STATE;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   LEMC_TRY(launch_basis(static_cast<const float2*>(rec_p), W, c->K, c->N, c->bprog,
-                        static_cast<float*>(V), ldv, nullptr, nullptr, st));
+                        static_cast<float*>(V), ldv, nullptr, nullptr, RangeOut{}, st));
   return order_after(c, st);
 }
 
@@ -1505,7 +1570,7 @@ int lemc_gram_device(lemc_ctx* c, const void* V, const void* rec_w, int W, int l
   LEMC_CUDA(cudaEventRecord(c->ev[2], user));
   LEMC_CUDA(cudaStreamWaitEvent(c->stream, c->ev[2], 0));
   LEMC_TRY(gram_step(c, static_cast<const float*>(V), static_cast<const float*>(rec_w), ldv, W,
-                     mode));
+                     mode, false));
   LEMC_CUDA(cudaEventRecord(c->ev[3], c->stream));
   LEMC_CUDA(cudaStreamWaitEvent(user, c->ev[3], 0));
   return LEMC_OK;

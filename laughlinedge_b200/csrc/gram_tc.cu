@@ -1,51 +1,63 @@
 // S/H contraction on the 5th-generation tensor cores (tcgen05, sm_100a).
 //
-// For every tile job (A panel of 128 V rows, B panel of 32 V rows, walker
+// For every job (A panel of 128 V rows, B panel of NB = 32 or 64 V rows, walker
 // split) the kernel accumulates
-//   D[r][h*32 + c] = sum_w V[a0+r][w] * W_h(w) * V[b0+c][w],   h = 0,1,2
-// with W_0 = w1, W_1 = w1 sum|z|^2, W_2 = w1 sum|z|^4: one M=128 x N=96 MMA
-// produces the S, H2 and H4 blocks at once.  Complex Gram entries are
+//   D[r][h*NB + c] = sum_w V[a0+r][w] * W_h(w) * V[b0+c][w],   h = 0,1,2
+// with W_0 = w1, W_1 = w1 sum|z|^2, W_2 = w1 sum|z|^4: one set of M=128 x N=3 NB
+// MMAs produces the S, H2 and H4 blocks at once.  Complex Gram entries are
 // recovered from the real products of the [Re; Im] row planes afterwards.
 //
-// Precision: each FP32 operand x is split x = hi + lo with hi = bf16(x),
-// lo = bf16(x - hi) (kind::f16) or hi = tf32_rn(x), lo = tf32_rn(x - hi)
-// (kind::tf32).  Each accumulator buffer holds 192 FP32 columns: hi*hi in the
-// first 96 and the correction products hi*lo + lo*hi (+ lo*lo) in the next 96.
-// One M=128 x N=192 MMA multiplies A_hi by the stacked [B_hi; B_lo] operand
-// (both products at once) and one N=96 MMA adds A_lo * B_hi to the
-// corrections.  A tcgen05.mma of kind::tf32 with K=8 costs about 97 cycles for
-// any N up to 128 and 106 cycles at N=192 (measured on B200), so this takes
-// 203 cycles per K step where three N=96 MMAs took 290.  The tensor core's
-// accumulation truncates (a relative bias of about -4e-8 per MMA step), so
-// every `flush_every` K-chunks the epilogue warps move both halves of the
-// buffer out of tensor memory into FP32 register sums (round-to-nearest; two
-// buffers let the MMAs continue meanwhile).  At the end each job adds its
-// sums, in FP64, to its private slot in global memory.
+// Precision: each FP32 operand x is split x = hi + lo into two 16-bit terms,
+// FP16 for LEMC_GRAM_TF32X3 (11 + 11 significant bits, as two TF32 terms carry, at
+// twice their MMA rate and half their operand bytes) or BF16, and the products
+// hi*hi + hi*lo + lo*hi (+ lo*lo) are summed.  FP16's range is met by a power-of-two
+// scale per V row and per weight plane, from the row's largest magnitude (a bound
+// on it, see row_bound_kernel), which puts the row's top at 2^15; terms below
+// 2^-25 of that scale are lost, i.e. 2^-40 of the row's largest value, where a
+// row's root mean square is at least its largest value over sqrt(walkers).  The
+// scales are undone in FP64.  Measured against FP64 sums of the same V (largest
+// normalised entry; FP16 here, TF32 before): N=50, 65536 walkers 4.9e-7, 5.6e-7;
+// N=200, 8192 walkers 5.7e-7, 7.5e-7; N=100, 16384 walkers 8.6e-7, 9.3e-7.
+// The tensor core's accumulation truncates (about -4e-8 per MMA step), so every
+// `flush_every` K-chunks (default one: 64 walkers, four steps) the epilogue warps
+// move the accumulators out of tensor memory into FP32 register sums
+// (round-to-nearest; two buffers let the MMAs continue meanwhile).  NB = 32 keeps
+// the corrections in columns of their own; NB = 64 has no room for them and adds
+// them first, while the accumulator is small.  At the end each job adds its sums,
+// in FP64, to its private slot in global memory.
+//
+// MMA shape: with A in tensor memory an MMA costs about 97 cycles for any N up to
+// 128 and 106 at N=192, so NB = 64 issues three N=192 MMAs a K step and NB = 32 one
+// N=192 (A_hi times the stacked [B_hi; B_lo]) and one N=96.
 //
 // Operand placement.  The A operand (hi and lo, 128 rows x one K-chunk) lives
 // in tensor memory: the A converters write it with tcgen05.st and the MMAs
 // read it from there, so shared memory only carries the raw TMA stages and
 // the (weighted, split) B operand.
 //
-// Pipeline (608 threads, one CTA per SM):
-//   warp 17      loader: tiled TMA loads per K-chunk (A panel 128 x KC in
-//                128-byte-swizzled boxes of 32 samples, B panel 32 x KC,
-//                weight planes 3 x KC; rows past the end are zero-filled by
-//                the TMA unit) into a ring of raw FP32 stages;
-//   warps 8-11   A converters: thread = A row (TMEM lane); raw FP32 -> hi/lo,
-//                stored to the tensor-memory A stage with tcgen05.st;
-//   warps 12-15  B converters: raw FP32 -> weighted, split hi/lo B operands in
+// Pipeline (896 threads, one CTA per SM, register shares moved by setmaxnreg):
+//   warp 25      loader: tiled TMA loads per half K-chunk of 32 walkers (A panel,
+//                B panel in 128-byte-swizzled rows, weight planes; rows past the
+//                end are zero-filled by the TMA unit) into a ring of raw stages;
+//   warps 8-15   A converters: thread = A row (TMEM lane) of one half of every
+//                chunk; raw FP32 -> scaled hi/lo, stored with tcgen05.st;
+//   warps 16-23  B converters: raw FP32 -> weighted, split hi/lo B operands in
 //                128-byte-swizzled K-major shared-memory layout;
-//   warp 16      allocates 512 TMEM columns, one lane issues tcgen05.mma;
-//   warp 18      scheduler: makes the issuer's barrier waits and hands each
+//   warp 24      allocates 512 TMEM columns, one lane issues tcgen05.mma;
+//   warp 26      scheduler: makes the issuer's barrier waits and hands each
 //                K-chunk to it through a named barrier;
-// (Doubling the converter warps to 864 threads held the kernel to 72
-// registers and ran slower: 0.321 against 0.266 ms at the mixed-precision
-// workload.)
-//   warps 0-7    epilogue: TMEM lane quarter = warp % 4, column half =
-//                warp / 4, 48 FP32 accumulators per thread.
-// Tensor memory columns: accumulator buffers at 0 and 192 (hi*hi at +0,
-// corrections at +96), A stages at 384 and 448 (hi at +0, lo at +32).
+//   warps 0-7    epilogue: TMEM lane quarter = warp % 4, column half = warp / 4.
+// Tensor memory columns: accumulator buffers at 0 and 192, A stages at 384 and
+// 448 (hi at +0, lo at +32).
+//
+// What bounds it: shared-memory bandwidth.  A 64-walker chunk at NB = 64 moves
+// about 217 KB through it (TMA writes 49, converter reads 48, B operands 48 written
+// and 72 read by the MMAs), 1700 cycles at 128 B/cycle against 1285 of MMA issue
+// and about 2700 measured; feeding the loads from L2 alone changes nothing.
+// Measured (B200, 65536 walkers): 2713 states 6.75 -> 3.0 ms, 526 states 0.76 ->
+// 0.39 ms, 272 states (NB = 32) 0.256 -> 0.152 ms.  One converter warp per scheduler
+// and operand: 4.1 ms; shared memory through generic pointers: 3.4 ms; slot updates
+// by each thread along its own row: 0.2 ms a job.
 // No load uses cluster multicast; every source is this GPU's own memory.
 // Every mbarrier wait is bounded in time; on expiry the kernel records
 // LEMC_ERR_TIMEOUT in the error word, skips its output and unwinds: the loader
@@ -53,6 +65,7 @@
 // the MMAs it has committed, then the CTA frees its tensor memory and exits.
 #include <cuda.h>
 #include <cuda_bf16.h>
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -62,54 +75,62 @@ namespace lemc {
 namespace {
 
 constexpr int kM = 128;            // A panel rows (MMA M)
-constexpr int kNB = 32;            // B panel rows per weight
-constexpr int kN = 3 * kNB;        // MMA N
+constexpr int kPanel = 32;         // B rows of one tile of the tile list
+constexpr int kPanelCols = 3 * kPanel;  // its output columns: [weight][row]
+constexpr int KC = 64;             // samples per K-chunk: one 128-byte operand row
+constexpr int kHalf = 32;          // samples per raw stage (half a K-chunk)
 constexpr int kOpRowBytes = 128;   // one swizzle-128B row of split operands
-constexpr int kBTileBytes = kN * kOpRowBytes;  // 12 KB
 constexpr int kOpStages = 2;
 constexpr int kEpiWarps = 8;
-constexpr int kAConvWarp0 = 8;     // warps 8-11: A converters (lane quarter = warp % 4)
-constexpr int kBConvWarp0 = 12;    // warps 12-15: B converters
-constexpr int kBConvThreads = 4 * 32;
-constexpr int kConvThreads = 8 * 32;
-constexpr int kEpiCols = kN / (kEpiWarps / 4);  // accumulator columns per epilogue thread
-constexpr int kMmaWarp = 16;
-constexpr int kLoadWarp = 17;
-constexpr int kSchedWarp = 18;     // does the issuer's barrier waits (see the MMA issuer)
-constexpr int kThreads = 19 * 32;
+constexpr int kAConvWarp0 = 8;     // warps 8-15: A converters (lane quarter = warp % 4)
+constexpr int kBConvWarp0 = 16;    // warps 16-23: B converters
+constexpr int kRawReaders = 8;     // converter warps that read one raw stage (4 A, 4 B)
+constexpr int kConvWarps = 16;     // converter warps that fill one operand stage
+constexpr int kMmaWarp = 24;
+constexpr int kLoadWarp = 25;
+constexpr int kSchedWarp = 26;     // does the issuer's barrier waits (see the MMA issuer)
+constexpr int kThreads = 28 * 32;  // seven warpgroups; warp 27 only fills the last one
+// Register shares after the roles split (setmaxnreg): 896 threads start with 72
+// each, and 256 x 120 + 512 x 56 + 128 x 40 = 896 x 72.
+constexpr int kLaunchRegs = 72, kEpiRegs = 120, kConvRegs = 56, kMiscRegs = 40;
+static_assert(256 * kEpiRegs + 512 * kConvRegs + 128 * kMiscRegs <= kThreads * kLaunchRegs,
+              "register split exceeds the launch's registers");
 constexpr int kTmemCols = 512;
-constexpr uint32_t kColBuf = 0;    // accumulator buffers at 0 and 192 (hi*hi +0, corrections +96)
-constexpr uint32_t kBufCols = 2 * kN;
+constexpr uint32_t kBufCols = 192; // accumulator buffers at columns 0 and 192
 constexpr uint32_t kColA = 384;    // A stages at 384 + 64 s (hi +0, lo +32)
 static_assert(2 * kBufCols <= kColA, "accumulator buffers overlap the A stages");
 constexpr long long kWaitCycles = 4000000000LL;  // default wait bound, ~2 s at 1.9 GHz
 
-template <bool TF32>
+// NB = B rows of a job: 64 (two adjacent tiles) or 32 (one).
+template <int NB>
 struct Cfg {
-  static constexpr int KC = TF32 ? 32 : 64;           // samples per K-chunk
-  static constexpr int RAW_ROW = KC * 4;              // bytes of one raw FP32 row segment
-  static constexpr int A_BOXES = KC / 32;             // 128-byte-wide swizzled A boxes
-  static constexpr int A_BYTES = kM * RAW_ROW;        // raw A (all boxes)
-  static constexpr int B_BYTES = kNB * RAW_ROW;
-  static constexpr int W_BYTES = 3 * KC * 4;
+  static constexpr int N = 3 * NB;                      // output columns
+  static constexpr int B_TILE = N * kOpRowBytes;        // bytes of the hi (or lo) B operand
+  static constexpr int A_BYTES = kM * kHalf * 4;
+  static constexpr int B_BYTES = NB * kHalf * 4;
+  static constexpr int W_BYTES = 3 * kHalf * 4;
   static constexpr int RAW_STAGE = A_BYTES + B_BYTES + 1024;  // weights padded to 1 KB
-  static constexpr int RAW_STAGES = TF32 ? 6 : 3;
+  static constexpr int RAW_STAGES = NB == 64 ? 5 : 8;
 };
 
-template <bool TF32>
+template <int NB>
 struct Smem {
-  uint8_t raw[Cfg<TF32>::RAW_STAGES][Cfg<TF32>::RAW_STAGE];  // 1024-aligned stages
-  uint8_t bop[kOpStages][2 * kBTileBytes];                    // B hi | B lo
-  uint64_t raw_full[Cfg<TF32>::RAW_STAGES];
-  uint64_t raw_empty[Cfg<TF32>::RAW_STAGES];
+  uint8_t raw[Cfg<NB>::RAW_STAGES][Cfg<NB>::RAW_STAGE];  // 1024-aligned stages
+  uint8_t bop[kOpStages][2 * Cfg<NB>::B_TILE];           // B hi | B lo
+  uint64_t raw_full[Cfg<NB>::RAW_STAGES];
+  uint64_t raw_empty[Cfg<NB>::RAW_STAGES];
   uint64_t op_full[kOpStages];
   uint64_t op_empty[kOpStages];
   uint64_t acc_full[2];
   uint64_t acc_empty[2];
   uint64_t done;
+  int row_exp[kM];                // scale exponents of the A rows and output columns
+  int col_exp[Cfg<NB>::N];
   uint32_t tmem_base;
   int abort_flag;
 };
+static_assert(sizeof(float) * kM * (Cfg<64>::N + 1) <= sizeof(Smem<64>::raw) &&
+                  sizeof(float) * kM * (Cfg<32>::N + 1) <= sizeof(Smem<32>::raw), "output staging");
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -140,14 +161,17 @@ __device__ __forceinline__ void named_sync(int id) {
   asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory");
 }
 
+// One test of a barrier phase; the hardware may suspend the thread up to the hint,
+// which keeps the waiting warps from filling the issue slots with polls.
+constexpr uint32_t kWaitHintNs = 20000;
 __device__ __forceinline__ bool mbar_try(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
+      : "r"(smem_u32(bar)), "r"(parity), "r"(kWaitHintNs)
       : "memory");
   return ok != 0;
 }
@@ -157,8 +181,17 @@ __device__ __forceinline__ bool mbar_try(uint64_t* bar, uint32_t parity) {
 // role gave up.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* abort_flag, int* err,
                                           long long limit) {
+  // a few tests for each look at the clock and the flag: up to two dozen warps
+  // wait at a time, and their polls take issue slots from the converters
+  auto test = [&]() {
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (mbar_try(bar, parity)) return true;
+    return false;
+  };
+  if (test()) return true;
   const long long t0 = clock64();
-  while (!mbar_try(bar, parity)) {
+  while (!test()) {
     if (*(volatile int*)abort_flag) return false;
     if (clock64() - t0 > limit) {
       *(volatile int*)abort_flag = 1;
@@ -211,23 +244,14 @@ __host__ __device__ constexpr uint32_t make_idesc(uint32_t ab_format, int n) {
          (uint32_t(kM >> 4) << 24);
 }
 
-// D (TMEM) += A (TMEM, 128 lanes x K) * B (shared memory descriptor)
-template <bool TF32>
+// D (TMEM) += A (TMEM, 128 lanes x K) * B (shared memory descriptor), 16-bit operands
 __device__ __forceinline__ void mma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc,
                                        uint32_t idesc, uint32_t accumulate) {
-  if (TF32) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
-        "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate));
-  } else {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
-        "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate));
-  }
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
+      "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate));
 }
 
 // 16 consecutive 32-bit columns of this thread's TMEM lane
@@ -260,11 +284,14 @@ __device__ __forceinline__ void fence_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t* r) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]),
-                 "=r"(r[6]), "=r"(r[7])
-               : "r"(taddr));
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+        "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr));
 }
 __device__ __forceinline__ void tmem_wait_ld() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -275,41 +302,41 @@ __device__ __forceinline__ uint32_t sw128_off(int r, int c) {
   return uint32_t((r >> 3) * 1024 + (r & 7) * 128 + ((c ^ (r & 7)) << 4));
 }
 
-__device__ __forceinline__ void split_bf16x8(const float* x, uint4& hi, uint4& lo) {
-  uint32_t h[4], l[4];
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const __nv_bfloat162 hb = __floats2bfloat162_rn(x[2 * q], x[2 * q + 1]);
-    const float2 hf = __bfloat1622float2(hb);
-    const __nv_bfloat162 lb = __floats2bfloat162_rn(x[2 * q] - hf.x, x[2 * q + 1] - hf.y);
-    h[q] = *reinterpret_cast<const uint32_t*>(&hb);
-    l[q] = *reinterpret_cast<const uint32_t*>(&lb);
+// Two samples x0, x1 as packed 16-bit pairs hi + lo: hi = x rounded to nearest,
+// lo = x - hi (exact in FP32) rounded to nearest.  FP16 (22 significant bits) or
+// BF16 (16).
+template <bool HALF>
+__device__ __forceinline__ void split2(float2 x, uint32_t& hi, uint32_t& lo) {
+  const float2 m1 = make_float2(-1.f, -1.f);
+  if (HALF) {
+    const __half2 h = __float22half2_rn(x);
+    const float2 r = __ffma2_rn(__half22float2(h), m1, x);  // x - hi, exact
+    const __half2 l = __float22half2_rn(r);
+    hi = *reinterpret_cast<const uint32_t*>(&h);
+    lo = *reinterpret_cast<const uint32_t*>(&l);
+  } else {
+    const __nv_bfloat162 h = __float22bfloat162_rn(x);
+    const float2 r = __ffma2_rn(__bfloat1622float2(h), m1, x);
+    const __nv_bfloat162 l = __float22bfloat162_rn(r);
+    hi = *reinterpret_cast<const uint32_t*>(&h);
+    lo = *reinterpret_cast<const uint32_t*>(&l);
   }
-  hi = make_uint4(h[0], h[1], h[2], h[3]);
-  lo = make_uint4(l[0], l[1], l[2], l[3]);
 }
 
-// x rounded to the nearest TF32 value (ties away from zero), as a 32-bit
-// pattern whose 13 low mantissa bits are zero.  Adding half a TF32 ulp to the
-// magnitude bits and truncating is that rounding for every finite x (a carry
-// into the exponent is the correct round-up; overflow gives infinity) and
-// runs as two integer ops at full ALU rate.
-__device__ __forceinline__ uint32_t to_tf32_rn(float x) {
-  return (__float_as_uint(x) + 0x1000u) & 0xFFFFE000u;
+// Power-of-two scales: a row (or weight plane) whose largest magnitude has the
+// FP32 bits `max_bits` is multiplied by 2^row_exp, which brings the maximum into
+// [2^14, 2^15) (weights: below 1), inside FP16's range; both steps and the
+// division afterwards are exact.  A zero row keeps 1; an infinite or NaN one
+// stays non-finite.
+constexpr int kRowTop = 14;
+__device__ __forceinline__ int scale_exp(uint32_t max_bits, int top) {
+  if (max_bits == 0u) return 0;
+  const int k = top - (int(max_bits >> 23) - 127);
+  return max(-126, min(126, k));
 }
-
-// hi = x rounded to nearest TF32, lo = (x - hi) rounded to nearest TF32: both
-// roundings are unbiased (the tensor core would otherwise truncate the low 13
-// bits of each operand, a systematic -2^-22 relative bias on every product).
-__device__ __forceinline__ void split_tf32x4(const float* x, uint4& hi, uint4& lo) {
-  uint32_t h[4], l[4];
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    h[q] = to_tf32_rn(x[q]);
-    l[q] = to_tf32_rn(x[q] - __uint_as_float(h[q]));
-  }
-  hi = make_uint4(h[0], h[1], h[2], h[3]);
-  lo = make_uint4(l[0], l[1], l[2], l[3]);
+__device__ __forceinline__ float pow2f(int k) { return __uint_as_float(uint32_t(k + 127) << 23); }
+__device__ __forceinline__ double pow2d(int k) {
+  return __longlong_as_double((long long)(k + 1023) << 52);
 }
 
 struct TcArgs {
@@ -319,6 +346,7 @@ struct TcArgs {
   const float* rec_w;   // weight planes, stride ldw (256-byte aligned rows)
   int ldw;
   const TcTile* tiles;
+  const uint32_t* range;  // bits of max |V row| [total_rows], then of max |W_h| [3]
   double* partials;
   int n_chunks_total;   // K-chunks over the padded walker range
   int n_splits;
@@ -329,21 +357,29 @@ struct TcArgs {
   int hold_loads;         // test hook: the loader issues nothing (the waits then expire)
 };
 
-template <bool TF32>
+template <int R>
+__device__ __forceinline__ void regs_inc() {
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R));
+}
+template <int R>
+__device__ __forceinline__ void regs_dec() {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R));
+}
+
+template <bool HALF, int NB>
 __global__ void __launch_bounds__(kThreads, 1)
 gram_tc_kernel(const TcArgs a, const __grid_constant__ CUtensorMap tmA,
                const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmW) {
-  using C = Cfg<TF32>;
-  constexpr int KC = C::KC;
-  constexpr int EPC = TF32 ? 4 : 8;          // elements per 16-byte B operand chunk
-  constexpr int NKSTEP = kOpRowBytes / 32;   // one MMA consumes 32 bytes of K
-  constexpr uint32_t IDESC = make_idesc(TF32 ? 2u : 1u, kN);          // N=96
-  constexpr uint32_t IDESC2 = make_idesc(TF32 ? 2u : 1u, 2 * kN);     // N=192: [B_hi; B_lo]
+  using C = Cfg<NB>;
+  constexpr int NKSTEP = kOpRowBytes / 32;   // one MMA consumes 32 bytes (16 samples) of K
+  constexpr uint32_t IDESC = make_idesc(HALF ? 0u : 1u, C::N);
+  constexpr uint32_t IDESC2 = make_idesc(HALF ? 0u : 1u, 192);
   constexpr int RS = C::RAW_STAGES;
 
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  Smem<TF32>* sm = reinterpret_cast<Smem<TF32>*>(
-      (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  // aligned by an offset, not by rounding a pointer through an integer: that
+  // loses the address space, and every access becomes a generic one
+  Smem<NB>* sm = reinterpret_cast<Smem<NB>*>(smem_raw + (-smem_u32(smem_raw) & 1023u));
 
   const TcTile tile = a.tiles[blockIdx.x];
   const int warp = threadIdx.x >> 5;
@@ -358,19 +394,28 @@ gram_tc_kernel(const TcArgs a, const __grid_constant__ CUtensorMap tmA,
   if (threadIdx.x == 0) {
     for (int s = 0; s < RS; ++s) {
       mbar_init(&sm->raw_full[s], 1);
-      mbar_init(&sm->raw_empty[s], kConvThreads);
+      mbar_init(&sm->raw_empty[s], kRawReaders);
     }
     for (int s = 0; s < kOpStages; ++s) {
-      mbar_init(&sm->op_full[s], kConvThreads);
+      mbar_init(&sm->op_full[s], kConvWarps);
       mbar_init(&sm->op_empty[s], 1);
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&sm->acc_full[b], 1);
-      mbar_init(&sm->acc_empty[b], kEpiWarps * 32);
+      mbar_init(&sm->acc_empty[b], kEpiWarps);
     }
     mbar_init(&sm->done, 1);
     sm->abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (threadIdx.x < C::N) {
+    const int h = int(threadIdx.x) / NB, rb = tile.col0 + int(threadIdx.x) % NB;
+    const int eb = rb < a.total_rows ? scale_exp(a.range[rb], kRowTop) : 0;
+    sm->col_exp[threadIdx.x] = eb + scale_exp(a.range[a.total_rows + h], -1);
+  }
+  if (threadIdx.x < kM) {
+    const int row = tile.row0 + int(threadIdx.x);
+    sm->row_exp[threadIdx.x] = row < a.total_rows ? scale_exp(a.range[row], kRowTop) : 0;
   }
   if (warp == kMmaWarp) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
@@ -383,271 +428,327 @@ gram_tc_kernel(const TcArgs a, const __grid_constant__ CUtensorMap tmA,
   tc_fence_after();
   const uint32_t tmem = sm->tmem_base;
   int* abort_flag = &sm->abort_flag;
-
-  if (warp == kLoadWarp) {
-    // ------------------------------- loader --------------------------------
-    if (lane == 0) {
-      const uint32_t tx_bytes = uint32_t(C::A_BYTES + C::B_BYTES + C::W_BYTES);
-      int issued = 0;
-      for (int c = 0; c < nch && !a.hold_loads; ++c) {
-        const int s = c % RS;
-        if (!mbar_wait(&sm->raw_empty[s], (uint32_t(c / RS) & 1u) ^ 1u, abort_flag, a.err, a.wait_cycles)) break;
-        const int k0 = (c_beg + c) * KC;
-        uint8_t* dst = sm->raw[s];
-        mbar_arrive_tx(&sm->raw_full[s], tx_bytes);
-#pragma unroll
-        for (int j = 0; j < C::A_BOXES; ++j)
-          tma_load_2d(dst + j * (kM * 128), &tmA, k0 + 32 * j, tile.row0, &sm->raw_full[s]);
-        tma_load_2d(dst + C::A_BYTES, &tmB, k0, tile.col0, &sm->raw_full[s]);
-        tma_load_2d(dst + C::A_BYTES + C::B_BYTES, &tmW, k0, 0, &sm->raw_full[s]);
-        ++issued;
-      }
-      // the copies still in flight land before the CTA may exit, whatever the
-      // other roles did: the last one issued into each stage
-      for (int c = max(0, issued - RS); c < issued; ++c)
-        mbar_drain(&sm->raw_full[c % RS], uint32_t(c / RS) & 1u, a.err, a.wait_cycles);
-    }
+  // warp-uniform bounded wait
+  auto wait_all = [&](uint64_t* bar, uint32_t parity) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, a.err, a.wait_cycles)) != 0;
+  };
+  // one arrival per warp, after every lane's part is done
+  auto arrive_warp = [&](uint64_t* bar) {
     __syncwarp();
-  } else if (warp >= kAConvWarp0 && warp < kBConvWarp0) {
-    // ---------------------------- A converters -----------------------------
-    // Thread = A row r = TMEM lane; its raw row segment sits in 128-byte
-    // swizzled boxes (16-byte chunk j of row r at r*128 + ((j ^ (r & 7)) << 4)).
-    const int quarter = warp & 3;
-    const int r = quarter * 32 + lane;
-    const uint32_t lane_base = uint32_t(quarter * 32) << 16;
-    for (int c = 0; c < nch; ++c) {
-      const int rs = c % RS, os = c % kOpStages;
-      if (!mbar_wait(&sm->raw_full[rs], uint32_t(c / RS) & 1u, abort_flag, a.err, a.wait_cycles)) break;
-      if (!mbar_wait(&sm->op_empty[os], (uint32_t(c / kOpStages) & 1u) ^ 1u, abort_flag, a.err, a.wait_cycles)) break;
-      tc_fence_after();
-      const uint8_t* raw = sm->raw[rs];
-      const uint32_t a_hi = tmem + lane_base + kColA + uint32_t(os * 64);
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        // 16 TMEM columns: TF32 -> 16 samples, BF16 -> 32 samples (2 per column)
-        uint32_t hv[16], lv[16];
-        if (TF32) {
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const int j = half * 4 + q;
-            const float4 f = *reinterpret_cast<const float4*>(raw + r * 128 + ((j ^ (r & 7)) << 4));
-            const float x[4] = {f.x, f.y, f.z, f.w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              hv[4 * q + e] = to_tf32_rn(x[e]);
-              lv[4 * q + e] = to_tf32_rn(x[e] - __uint_as_float(hv[4 * q + e]));
-            }
-          }
-        } else {
-          const uint8_t* box = raw + half * (kM * 128);
-#pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            const float4 f = *reinterpret_cast<const float4*>(box + r * 128 + ((q ^ (r & 7)) << 4));
-            const float x[4] = {f.x, f.y, f.z, f.w};
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-              const __nv_bfloat162 hb = __floats2bfloat162_rn(x[2 * e], x[2 * e + 1]);
-              const float2 hf = __bfloat1622float2(hb);
-              const __nv_bfloat162 lb = __floats2bfloat162_rn(x[2 * e] - hf.x, x[2 * e + 1] - hf.y);
-              hv[2 * q + e] = *reinterpret_cast<const uint32_t*>(&hb);
-              lv[2 * q + e] = *reinterpret_cast<const uint32_t*>(&lb);
-            }
+    if (lane == 0) mbar_arrive(bar);
+  };
+
+  if (warp >= kMmaWarp) {
+    regs_dec<kMiscRegs>();
+    if (warp == kLoadWarp) {
+      // ------------------------------- loader ------------------------------
+      if (lane == 0) {
+        constexpr uint32_t tx_bytes = uint32_t(C::A_BYTES + C::B_BYTES + C::W_BYTES);
+        const int nh = 2 * nch;
+        int issued = 0, s = 0;
+        uint32_t ph = 1u;
+        for (int hc = 0; hc < nh && !a.hold_loads; ++hc) {
+          if (!mbar_wait(&sm->raw_empty[s], ph, abort_flag, a.err, a.wait_cycles)) break;
+          const int k0 = c_beg * KC + hc * kHalf;
+          uint8_t* dst = sm->raw[s];
+          mbar_arrive_tx(&sm->raw_full[s], tx_bytes);
+          tma_load_2d(dst, &tmA, k0, tile.row0, &sm->raw_full[s]);
+          tma_load_2d(dst + C::A_BYTES, &tmB, k0, tile.col0, &sm->raw_full[s]);
+          tma_load_2d(dst + C::A_BYTES + C::B_BYTES, &tmW, k0, 0, &sm->raw_full[s]);
+          ++issued;
+          if (++s == RS) {
+            s = 0;
+            ph ^= 1u;
           }
         }
-        tmem_st16(a_hi + half * 16, hv);
-        tmem_st16(a_hi + 32 + half * 16, lv);
+        // the copies still in flight land before the CTA may exit, whatever the
+        // other roles did: the last one issued into each stage
+        for (int hc = max(0, issued - RS); hc < issued; ++hc)
+          mbar_drain(&sm->raw_full[hc % RS], uint32_t(hc / RS) & 1u, a.err, a.wait_cycles);
       }
-      tmem_wait_st();
-      tc_fence_before();
-      mbar_arrive(&sm->op_full[os]);
-      mbar_arrive(&sm->raw_empty[rs]);
-    }
-  } else if (warp >= kBConvWarp0 && warp < kBConvWarp0 + 4) {
-    // ---------------------------- B converters -----------------------------
-    const int t = threadIdx.x - kBConvWarp0 * 32;
-    for (int c = 0; c < nch; ++c) {
-      const int rs = c % RS, os = c % kOpStages;
-      if (!mbar_wait(&sm->raw_full[rs], uint32_t(c / RS) & 1u, abort_flag, a.err, a.wait_cycles)) break;
-      if (!mbar_wait(&sm->op_empty[os], (uint32_t(c / kOpStages) & 1u) ^ 1u, abort_flag, a.err, a.wait_cycles)) break;
-      const uint8_t* rawb = sm->raw[rs] + C::A_BYTES;
-      const float* rw = reinterpret_cast<const float*>(sm->raw[rs] + C::A_BYTES + C::B_BYTES);
-      uint8_t* b_hi = sm->bop[os];
-      uint8_t* b_lo = b_hi + kBTileBytes;
-      // 32 rows x 8 operand chunks x 3 weight planes.  A thread's chunks share
-      // one column range (ch = t % 8), so the weight products are formed once
-      // per K-chunk and the independent chunks are interleaved.
-      constexpr int kItems = (kNB * 8) / kBConvThreads;
-      const int ch = t & 7;
-      float ww[3][EPC];
+      __syncwarp();
+    } else if (warp == kSchedWarp) {
+      // ----------------------------- scheduler -----------------------------
+      // An mbarrier test made by the thread that has just issued tcgen05.commit
+      // stalls until the committed MMAs retire, which drains the tensor pipe every
+      // K-chunk.  So this warp makes the issuer's waits (operand stage full;
+      // accumulator buffer empty at the start of a flush group) and hands each chunk
+      // over through a named barrier, which needs no shared-memory access.  It
+      // arrives once per chunk whatever happens (after an abort without
+      // waiting), so the issuer's barrier always completes.
+      int s = 0, b = 0, f = 0;
+      uint32_t ph_op = 0, ph_acc = 0;
+      for (int c = 0; c < nch; ++c) {
+        if (c >= 2) named_sync(3 + (c & 1));  // chunk c-2 issued: ids 1/2 are free again
+        if (lane == 0 && !*(volatile int*)abort_flag) {
+          bool ok = true;
+          if (f == 0) {
+            ok = mbar_wait(&sm->acc_empty[b], ((ph_acc >> b) & 1u) ^ 1u, abort_flag, a.err, a.wait_cycles);
+            ph_acc ^= 1u << b;
+          }
+          if (ok) mbar_wait(&sm->op_full[s], ph_op, abort_flag, a.err, a.wait_cycles);
+        }
+        __syncwarp();
+        named_arrive(1 + (c & 1));
+        if (++f == F || c == nch - 1) {
+          f = 0;
+          b ^= 1;
+        }
+        if (++s == kOpStages) {
+          s = 0;
+          ph_op ^= 1u;
+        }
+      }
+      for (int c = max(0, nch - 2); c < nch; ++c) named_sync(3 + (c & 1));
+    } else if (warp == kMmaWarp) {
+      // ---------------------------- MMA issuer -----------------------------
+      // One thread issues every MMA, so its per-MMA instruction count bounds the
+      // tensor-core issue rate: all descriptors and TMEM addresses are formed
+      // once per stage, a K step only adds a constant, and the flush schedule is
+      // kept in counters.  Its waits are made by the scheduler warp.
+      const bool four = a.passes > 3;
+      static_assert(kOpStages == 2, "the issuer keeps one descriptor per operand stage");
+      const uint64_t bdesc0 = sw128_desc(smem_u32(sm->bop[0]));
+      const uint64_t bdesc1 = sw128_desc(smem_u32(sm->bop[1]));
+      constexpr uint64_t kLoDesc = uint64_t(C::B_TILE >> 4);  // B lo tile, in descriptor units
+      int s = 0, b = 0, f = 0;          // operand stage, accumulator buffer, chunk within flush group
+      int issued = 0;
+      for (int c = 0; c < nch; ++c) {
+        named_sync(1 + (c & 1));
+        const bool go = !*(volatile int*)abort_flag;
+        if (lane == 0 && go) {
+          tc_fence_after();
+          const uint64_t bh = s ? bdesc1 : bdesc0, bl = bh + kLoDesc;
+          const uint32_t ahi = tmem + kColA + uint32_t(s * 64), alo = ahi + 32;
+          const uint32_t d = tmem + uint32_t(b) * kBufCols;
+          // the first MMA of a flush group overwrites the buffer.  K step ks: B
+          // advances 32 bytes (2 descriptor units), A 8 TMEM columns
+          const uint32_t acc_d = f == 0 ? 0u : 1u;
+          if constexpr (NB == 64) {
+            // the small products first, while the accumulator is small
 #pragma unroll
-      for (int e = 0; e < EPC; ++e) {
-        const float one = rw[ch * EPC + e];
-        ww[0][e] = one;
-        ww[1][e] = one * rw[KC + ch * EPC + e];
-        ww[2][e] = one * rw[2 * KC + ch * EPC + e];
+            for (int ks = 0; ks < NKSTEP; ++ks) {
+              mma_ts(d, ahi + 8 * ks, bl + 2 * ks, IDESC, ks == 0 ? acc_d : 1u);
+              mma_ts(d, alo + 8 * ks, bh + 2 * ks, IDESC, 1u);
+              if (four) mma_ts(d, alo + 8 * ks, bl + 2 * ks, IDESC, 1u);
+            }
+#pragma unroll
+            for (int ks = 0; ks < NKSTEP; ++ks) mma_ts(d, ahi + 8 * ks, bh + 2 * ks, IDESC, 1u);
+          } else {
+            // hi*hi | corrections side by side; the B hi and lo tiles are
+            // contiguous, so bh with N=192 spans both
+            const uint32_t dc = d + C::N;
+#pragma unroll
+            for (int ks = 0; ks < NKSTEP; ++ks) {
+              mma_ts(d, ahi + 8 * ks, bh + 2 * ks, IDESC2, ks == 0 ? acc_d : 1u);
+              mma_ts(dc, alo + 8 * ks, bh + 2 * ks, IDESC, 1u);
+              if (four) mma_ts(dc, alo + 8 * ks, bl + 2 * ks, IDESC, 1u);
+            }
+          }
+          umma_commit(&sm->op_empty[s]);
+          if (f + 1 == F || c == nch - 1) umma_commit(&sm->acc_full[b]);
+          ++issued;
+        }
+        __syncwarp();
+        named_arrive(3 + (c & 1));
+        if (++f == F || c == nch - 1) {
+          f = 0;
+          b ^= 1;
+        }
+        if (++s == kOpStages) s = 0;
       }
-      float x[kItems][EPC];
+      if (lane == 0 && issued > 0) {
+        // every issued MMA must retire before TMEM is released
+        umma_commit(&sm->done);
+        mbar_drain(&sm->done, 0u, a.err, a.wait_cycles);
+      }
+      __syncwarp();
+    }
+  } else if (warp >= kAConvWarp0) {
+    // Four warps of each kind take the first half of every K-chunk, four the
+    // second: one warp per scheduler and operand is latency-bound (about five
+    // cycles an instruction), 2330 cycles a chunk for B against 1370 of MMAs.
+    regs_dec<kConvRegs>();
+    const int half = (warp >> 2) & 1;
+    int rs = half;  // raw stage of (chunk c, half): 2 c + half
+    uint32_t ph_raw = 0u, ph_op = 1u;
+    if (warp < kBConvWarp0) {
+      // --------------------------- A converters ----------------------------
+      // Thread = A row r = TMEM lane; its raw row segment is a 128-byte
+      // swizzled row (16-byte chunk j of row r at r*128 + ((j ^ (r & 7)) << 4)).
+      const int quarter = warp & 3;
+      const int r = quarter * 32 + lane;
+      const uint32_t a_col = tmem + (uint32_t(quarter * 32) << 16) + kColA + uint32_t(half * 16);
+      const float sc1 = pow2f(sm->row_exp[r]);
+      const float2 sc = make_float2(sc1, sc1);
+      for (int c = 0; c < nch; ++c) {
+        const int os = c & 1;
+        if (!wait_all(&sm->raw_full[rs], ph_raw)) break;
+        const uint8_t* raw = sm->raw[rs] + r * 128;
+        // 16 TMEM columns of 2 samples each
+        uint32_t hv[16], lv[16];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const float4 f = *reinterpret_cast<const float4*>(raw + ((q ^ (r & 7)) << 4));
+          split2<HALF>(__fmul2_rn(make_float2(f.x, f.y), sc), hv[2 * q], lv[2 * q]);
+          split2<HALF>(__fmul2_rn(make_float2(f.z, f.w), sc), hv[2 * q + 1], lv[2 * q + 1]);
+        }
+        arrive_warp(&sm->raw_empty[rs]);
+        if ((rs += 2) >= RS) {
+          rs -= RS;
+          ph_raw ^= 1u;
+        }
+        if (!wait_all(&sm->op_empty[os], ph_op)) break;
+        ph_op ^= uint32_t(os);
+        tc_fence_after();
+        tmem_st16(a_col + uint32_t(os * 64), hv);
+        tmem_st16(a_col + uint32_t(os * 64) + 32, lv);
+        tmem_wait_st();
+        tc_fence_before();
+        arrive_warp(&sm->op_full[os]);
+      }
+    } else {
+      // --------------------------- B converters ----------------------------
+      // NB rows x 4 operand chunks (8 samples) x 3 weight planes per raw stage.
+      // A thread's items share one column range, so the weight products are
+      // formed once; eight consecutive lanes hold eight rows of one chunk, which
+      // the 128-byte swizzle spreads over all banks, reading and writing.
+      const int t = threadIdx.x & 127;
+      constexpr int kItems = NB / 32;
+      const int ch = (t >> 3) & 3, rb0 = (t & 7) + 8 * (t >> 5);
+      float sc[kItems], ws[3];
 #pragma unroll
       for (int q = 0; q < kItems; ++q) {
-        const int rb = (q * kBConvThreads + t) >> 3;
-        const float4* src = reinterpret_cast<const float4*>(rawb + rb * C::RAW_ROW + ch * EPC * 4);
-#pragma unroll
-        for (int v = 0; v < EPC / 4; ++v) {
-          const float4 f = src[v];
-          x[q][4 * v] = f.x; x[q][4 * v + 1] = f.y; x[q][4 * v + 2] = f.z; x[q][4 * v + 3] = f.w;
-        }
+        const int row = tile.col0 + rb0 + 32 * q;
+        sc[q] = pow2f(row < a.total_rows ? scale_exp(a.range[row], kRowTop) : 0);
       }
 #pragma unroll
-      for (int h = 0; h < 3; ++h) {
+      for (int h = 0; h < 3; ++h) ws[h] = pow2f(scale_exp(a.range[a.total_rows + h], -1));
+      for (int c = 0; c < nch; ++c) {
+        const int os = c & 1;
+        if (!wait_all(&sm->op_empty[os], ph_op)) break;
+        ph_op ^= uint32_t(os);
+        uint8_t* b_hi = sm->bop[os];
+        uint8_t* b_lo = b_hi + C::B_TILE;
+        if (!wait_all(&sm->raw_full[rs], ph_raw)) break;
+        const uint8_t* rawb = sm->raw[rs] + C::A_BYTES;
+        const float4* rw = reinterpret_cast<const float4*>(rawb + C::B_BYTES) + 2 * ch;
+        float2 x[kItems][4];
 #pragma unroll
         for (int q = 0; q < kItems; ++q) {
-          const int rb = (q * kBConvThreads + t) >> 3;
-          float y[EPC];
+          const int rb = rb0 + 32 * q;
+          const float2 sq = make_float2(sc[q], sc[q]);
 #pragma unroll
-          for (int e = 0; e < EPC; ++e) y[e] = x[q][e] * ww[h][e];
-          uint4 hi, lo;
-          if (TF32) split_tf32x4(y, hi, lo); else split_bf16x8(y, hi, lo);
-          const uint32_t off = sw128_off(h * kNB + rb, ch);
-          *reinterpret_cast<uint4*>(b_hi + off) = hi;
-          *reinterpret_cast<uint4*>(b_lo + off) = lo;
+          for (int v = 0; v < 2; ++v) {
+            const float4 g = *reinterpret_cast<const float4*>(
+                rawb + rb * 128 + (((2 * ch + v) ^ (rb & 7)) << 4));
+            x[q][2 * v] = __fmul2_rn(make_float2(g.x, g.y), sq);
+            x[q][2 * v + 1] = __fmul2_rn(make_float2(g.z, g.w), sq);
+          }
         }
-      }
-      fence_async_smem();
-      mbar_arrive(&sm->op_full[os]);
-      mbar_arrive(&sm->raw_empty[rs]);
-    }
-  } else if (warp == kSchedWarp) {
-    // ------------------------------ scheduler -------------------------------
-    // An mbarrier test made by the thread that has just issued tcgen05.commit
-    // stalls until the committed MMAs retire, which drains the tensor pipe every
-    // K-chunk.  So this warp makes the issuer's waits (operand stage full;
-    // hi*hi buffer empty at the start of a flush group) and hands each chunk
-    // over through a named barrier, which needs no shared-memory access.  It
-    // arrives once per chunk whatever happens (after an abort without
-    // waiting), so the issuer's barrier always completes.
-    int s = 0, b = 0, f = 0;
-    uint32_t ph_op = 0, ph_acc = 0;
-    for (int c = 0; c < nch; ++c) {
-      if (c >= 2) named_sync(3 + (c & 1));  // chunk c-2 issued: ids 1/2 are free again
-      if (lane == 0 && !*(volatile int*)abort_flag) {
-        bool ok = true;
-        if (f == 0) {
-          ok = mbar_wait(&sm->acc_empty[b], ((ph_acc >> b) & 1u) ^ 1u, abort_flag, a.err, a.wait_cycles);
-          ph_acc ^= 1u << b;
-        }
-        if (ok) mbar_wait(&sm->op_full[s], ph_op, abort_flag, a.err, a.wait_cycles);
-      }
-      __syncwarp();
-      named_arrive(1 + (c & 1));
-      if (++f == F || c == nch - 1) {
-        f = 0;
-        b ^= 1;
-      }
-      if (++s == kOpStages) {
-        s = 0;
-        ph_op ^= 1u;
-      }
-    }
-    for (int c = max(0, nch - 2); c < nch; ++c) named_sync(3 + (c & 1));
-  } else if (warp == kMmaWarp) {
-    // ------------------------------ MMA issuer -----------------------------
-    // One thread issues every MMA, so its per-MMA instruction count bounds the
-    // tensor-core issue rate: all descriptors and TMEM addresses are formed
-    // once per stage, a K step only adds a constant, and the flush schedule is
-    // kept in counters.  Its waits are made by the scheduler warp.
-    const bool four = a.passes > 3;
-    static_assert(kOpStages == 2, "the issuer keeps one descriptor per operand stage");
-    const uint64_t bdesc0 = sw128_desc(smem_u32(sm->bop[0]));
-    const uint64_t bdesc1 = sw128_desc(smem_u32(sm->bop[1]));
-    constexpr uint64_t kLoDesc = uint64_t(kBTileBytes >> 4);  // B lo tile, in descriptor units
-    int s = 0, b = 0, f = 0;          // operand stage, hi*hi buffer, chunk within flush group
-    int issued = 0;
-    for (int c = 0; c < nch; ++c) {
-      named_sync(1 + (c & 1));
-      const bool go = !*(volatile int*)abort_flag;
-      if (lane == 0 && go) {
-        tc_fence_after();
-        const uint64_t bh = s ? bdesc1 : bdesc0, bl = bh + kLoDesc;
-        const uint32_t ahi = tmem + kColA + uint32_t(s * 64), alo = ahi + 32;
-        const uint32_t d = tmem + kColBuf + uint32_t(b) * kBufCols;  // hi*hi | corrections
-        const uint32_t dc = d + kN;
-        // the first MMA of a flush group overwrites both halves of the buffer
-        const uint32_t acc_d = f == 0 ? 0u : 1u;
-        // K step ks: B advances 32 bytes (2 descriptor units), A 8 TMEM columns;
-        // the B hi and lo tiles are contiguous, so bh with N=192 spans both
-        mma_ts<TF32>(d, ahi, bh, IDESC2, acc_d);
-        mma_ts<TF32>(dc, alo, bh, IDESC, 1u);
-        if (four) mma_ts<TF32>(dc, alo, bl, IDESC, 1u);
 #pragma unroll
-        for (int ks = 1; ks < NKSTEP; ++ks) {
-          mma_ts<TF32>(d, ahi + 8 * ks, bh + 2 * ks, IDESC2, 1u);
-          mma_ts<TF32>(dc, alo + 8 * ks, bh + 2 * ks, IDESC, 1u);
-          if (four) mma_ts<TF32>(dc, alo + 8 * ks, bl + 2 * ks, IDESC, 1u);
+        for (int h = 0; h < 3; ++h) {
+          const float2 wsh = make_float2(ws[h], ws[h]);
+          float2 ww[4];
+#pragma unroll
+          for (int v = 0; v < 2; ++v) {
+            const float4 o = rw[v];
+            ww[2 * v] = make_float2(o.x, o.y);
+            ww[2 * v + 1] = make_float2(o.z, o.w);
+            if (h > 0) {
+              const float4 f = rw[h * (kHalf / 4) + v];
+              ww[2 * v] = __fmul2_rn(ww[2 * v], make_float2(f.x, f.y));
+              ww[2 * v + 1] = __fmul2_rn(ww[2 * v + 1], make_float2(f.z, f.w));
+            }
+            ww[2 * v] = __fmul2_rn(ww[2 * v], wsh);
+            ww[2 * v + 1] = __fmul2_rn(ww[2 * v + 1], wsh);
+          }
+#pragma unroll
+          for (int q = 0; q < kItems; ++q) {
+            uint32_t hi[4], lo[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) split2<HALF>(__fmul2_rn(x[q][e], ww[e]), hi[e], lo[e]);
+            const uint32_t off = sw128_off(h * NB + rb0 + 32 * q, half * 4 + ch);
+            *reinterpret_cast<uint4*>(b_hi + off) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+            *reinterpret_cast<uint4*>(b_lo + off) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+          }
         }
-        umma_commit(&sm->op_empty[s]);
-        if (f + 1 == F || c == nch - 1) umma_commit(&sm->acc_full[b]);
-        ++issued;
+        arrive_warp(&sm->raw_empty[rs]);
+        if ((rs += 2) >= RS) {
+          rs -= RS;
+          ph_raw ^= 1u;
+        }
+        fence_async_smem();
+        arrive_warp(&sm->op_full[os]);
       }
-      __syncwarp();
-      named_arrive(3 + (c & 1));
-      if (++f == F || c == nch - 1) {
-        f = 0;
-        b ^= 1;
-      }
-      if (++s == kOpStages) s = 0;
     }
-    if (lane == 0 && issued > 0) {
-      // every issued MMA must retire before TMEM is released
-      umma_commit(&sm->done);
-      mbar_drain(&sm->done, 0u, a.err, a.wait_cycles);
-    }
-    __syncwarp();
-  } else if (warp < kEpiWarps) {
+  } else {
     // ------------------------------- epilogue ------------------------------
+    regs_inc<kEpiRegs>();
+    constexpr int EC = C::N / 2;                // output columns per thread
     const int quarter = warp & 3;
-    const int part0 = (warp >> 2) * kEpiCols;  // first accumulator column of this thread
+    const int part0 = (warp >> 2) * EC;         // first output column of this thread
     // Plain FP32 running sums (round-to-nearest, unbiased): over n flushes the
     // relative rounding error is ~2^-24 sqrt(n) / 3 per split, and the FP64
-    // sum over splits averages it down further.  Columns are read eight at a
-    // time to stay within the register budget.
-    float sum[kEpiCols];
+    // sum over splits averages it down further.
+    float2 sum[EC / 2];
 #pragma unroll
-    for (int i = 0; i < kEpiCols; ++i) sum[i] = 0.f;
+    for (int i = 0; i < EC / 2; ++i) sum[i] = make_float2(0.f, 0.f);
     const uint32_t lane_base = uint32_t(quarter * 32) << 16;
     bool ok = true;
     for (int q = 0; q < nint; ++q) {
       const int b = q & 1;
-      if (!mbar_wait(&sm->acc_full[b], uint32_t(q >> 1) & 1u, abort_flag, a.err, a.wait_cycles)) {
-        ok = false;
-        break;
-      }
+      if (!(ok = wait_all(&sm->acc_full[b], uint32_t(q >> 1) & 1u))) break;
       tc_fence_after();
-      // hi*hi column j and its correction column j + 96 belong to one sum
-      const uint32_t ta = tmem + lane_base + kColBuf + uint32_t(b) * kBufCols + uint32_t(part0);
+      const uint32_t ta = tmem + lane_base + uint32_t(b) * kBufCols + uint32_t(part0);
 #pragma unroll
-      for (int part = 0; part < kEpiCols / 8; ++part) {
-        uint32_t v0[8], v1[8];
-        tmem_ld8(ta + part * 8, v0);
-        tmem_ld8(ta + kN + part * 8, v1);
+      for (int part = 0; part < EC / 16; ++part) {
+        uint32_t v0[16], v1[16];
+        tmem_ld16(ta + part * 16, v0);
+        // NB == 32: column j's corrections sit at j + 96
+        if constexpr (NB == 32) tmem_ld16(ta + C::N + part * 16, v1);
         tmem_wait_ld();
-        if (part == kEpiCols / 8 - 1) {
+        if (part == EC / 16 - 1) {
           // every column of this buffer is in registers: the MMAs may reuse it
           tc_fence_before();
-          mbar_arrive(&sm->acc_empty[b]);
+          arrive_warp(&sm->acc_empty[b]);
         }
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          sum[part * 8 + i] += __uint_as_float(v0[i]);
-          sum[part * 8 + i] += __uint_as_float(v1[i]);
+          float2& t = sum[part * 8 + i];
+          t = __fadd2_rn(t, make_float2(__uint_as_float(v0[2 * i]), __uint_as_float(v0[2 * i + 1])));
+          if constexpr (NB == 32)
+            t = __fadd2_rn(t, make_float2(__uint_as_float(v1[2 * i]), __uint_as_float(v1[2 * i + 1])));
         }
       }
     }
-    if (ok && nch > 0) {
-      if (!*(volatile int*)abort_flag) {
-        double* slot = a.partials + (size_t)tile.slot * (kM * kN) +
-                       (size_t)(quarter * 32 + lane) * kN + part0;
+    // Stage the sums in the raw buffers (every copy into them has landed and been
+    // read once the last accumulator is full), then undo the scales (exact powers
+    // of two) in FP64 and add them to the slots along rows: a thread's own
+    // row-wise update touches 32 rows, 768 bytes apart, per warp access, and
+    // cost 60 us a job.
+    if (nch > 0) {
+      float* out = reinterpret_cast<float*>(sm->raw);
+      if (ok) {
+        float* mine = out + (quarter * 32 + lane) * (C::N + 1) + part0;
 #pragma unroll
-        for (int i = 0; i < kEpiCols; ++i) slot[i] += double(sum[i]);
+        for (int j = 0; j < EC / 2; ++j) {
+          mine[2 * j] = sum[j].x;
+          mine[2 * j + 1] = sum[j].y;
+        }
+      }
+      asm volatile("bar.sync 5, %0;" ::"n"(kEpiWarps * 32) : "memory");
+      if (ok && !*(volatile int*)abort_flag) {
+        double* slot = a.partials + (size_t)tile.slot * (kM * kPanelCols);
+#pragma unroll 4
+        for (int e = threadIdx.x; e < tile.panels * kM * kPanelCols; e += kEpiWarps * 32) {
+          const int i = (e / kPanelCols) % kM, j = e % kPanelCols;
+          const int col = j / kPanel * NB + e / (kM * kPanelCols) * kPanel + j % kPanel;  // [h][rb]
+          // one CTA per slot and launch: the reduction keeps the sum deterministic
+          // and needs no round trip to L2
+          atomicAdd(slot + e, double(out[i * (C::N + 1) + col]) *
+                                  pow2d(-(sm->row_exp[i] + sm->col_exp[col])));
+        }
       }
     }
   }
@@ -680,21 +781,21 @@ __global__ void gram_tc_reduce_kernel(const double* __restrict__ partials,
   const int a = idx / D, b = idx % D;
   auto C = [&](int r1, int r2, int h) {
     // A slice x holds B panels y >= 4 x only (the others are transposes)
-    if ((r2 - sc.b_base) / kNB < 4 * ((r1 - sc.a_base) / kM)) {
+    if ((r2 - sc.b_base) / kPanel < 4 * ((r1 - sc.a_base) / kM)) {
       const int r = r1;
       r1 = r2;
       r2 = r;
     }
-    const int x = (r1 - sc.a_base) / kM, y = (r2 - sc.b_base) / kNB;
+    const int x = (r1 - sc.a_base) / kM, y = (r2 - sc.b_base) / kPanel;
     const int t = sc.tile0 + x * sc.n_bpanels - 2 * x * (x - 1) + (y - 4 * x);
     double v = 0.0;
     if (t < 0 || t >= n_tiles) return v;
     const TcTile tl = tiles[t];
     const int i = r1 - tl.row0, j = r2 - tl.col0;
-    if (i < 0 || i >= kM || j < 0 || j >= kNB) return v;
+    if (i < 0 || i >= kM || j < 0 || j >= kPanel) return v;
     for (int sp = 0; sp < n_splits; ++sp) {
-      const double* slot = partials + (size_t)(sp * n_tiles + t) * (kM * kN);
-      v += slot[i * kN + h * kNB + j];
+      const double* slot = partials + (size_t)(sp * n_tiles + t) * (kM * kPanelCols);
+      v += slot[i * kPanelCols + h * kPanel + j];
     }
     return v;
   };
@@ -744,21 +845,52 @@ bool make_map(CUtensorMap* m, const float* base, int ld, int rows, int box_x, in
             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <bool TF32>
+template <bool HALF, int NB>
 int launch_t(const TcArgs& a, int n_jobs, cudaStream_t st) {
-  const size_t smem = sizeof(Smem<TF32>) + 1024;
+  const size_t smem = sizeof(Smem<NB>) + 1024;
   if (smem > 227 * 1024) return LEMC_ERR_CAPACITY;
-  constexpr int KC = Cfg<TF32>::KC;
   CUtensorMap tmA, tmB, tmW;
-  if (!make_map(&tmA, a.V, a.ldv, a.total_rows, 32, kM, true) ||
-      !make_map(&tmB, a.V, a.ldv, a.total_rows, KC, kNB, false) ||
-      !make_map(&tmW, a.rec_w, a.ldw, 3, KC, 3, false))
+  if (!make_map(&tmA, a.V, a.ldv, a.total_rows, kHalf, kM, true) ||
+      !make_map(&tmB, a.V, a.ldv, a.total_rows, kHalf, NB, true) ||
+      !make_map(&tmW, a.rec_w, a.ldw, 3, kHalf, 3, false))
     return LEMC_ERR_CUDA;
-  if (cudaFuncSetAttribute(gram_tc_kernel<TF32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  cudaFuncAttributes fa;
+  // the register split after launch assumes exactly kLaunchRegs per thread
+  if (cudaFuncGetAttributes(&fa, gram_tc_kernel<HALF, NB>) != cudaSuccess || fa.numRegs != kLaunchRegs ||
+      cudaFuncSetAttribute(gram_tc_kernel<HALF, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            int(smem)) != cudaSuccess)
     return LEMC_ERR_CUDA;
-  gram_tc_kernel<TF32><<<n_jobs, kThreads, smem, st>>>(a, tmA, tmB, tmW);
+  gram_tc_kernel<HALF, NB><<<n_jobs, kThreads, smem, st>>>(a, tmA, tmB, tmW);
   return cudaPeekAtLastError() == cudaSuccess ? LEMC_OK : LEMC_ERR_CUDA;
+}
+
+// range[r] = bits of max |V[r][w]| over the padded walkers, range[rows + h] of
+// max |W_h|, by unsigned maxima of the sign-cleared bits (NaN above infinity).
+// One read of V; the arrays were cleared before the launch.
+constexpr int kRangeThreads = 256, kRangeSpan = 8192;
+
+__global__ void __launch_bounds__(kRangeThreads)
+row_range_kernel(const float* __restrict__ V, int ldv, int rows, const float* __restrict__ rec_w,
+                 int ldw, int Wpad, uint32_t* __restrict__ range) {
+  const int r = blockIdx.y;
+  const int w0 = blockIdx.x * kRangeSpan, w1 = min(Wpad, w0 + kRangeSpan);
+  uint32_t m = 0u;
+  auto take = [&](float x) { m = max(m, __float_as_uint(x) & 0x7FFFFFFFu); };
+  if (r < rows) {
+    const float4* p = reinterpret_cast<const float4*>(V + (size_t)r * ldv);
+    for (int q = w0 / 4 + threadIdx.x; q < w1 / 4; q += kRangeThreads) {
+      const float4 f = p[q];
+      take(f.x); take(f.y); take(f.z); take(f.w);
+    }
+  } else {
+    const int h = r - rows;
+    for (int w = w0 + threadIdx.x; w < w1; w += kRangeThreads) {
+      const float one = rec_w[w];
+      take(h == 0 ? one : one * rec_w[(size_t)h * ldw + w]);
+    }
+  }
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) == 0 && m) atomicMax(range + r, m);
 }
 
 // Host-side settings of the bounded waits (lemc_debug_gram_wait).
@@ -775,15 +907,15 @@ int set_gram_wait(long long cycles, int hold_loads) {
 }
 
 int launch_gram_tc_rows(const float* V, int ldv, int total_rows, const float* rec_w, int ldw,
-                        int Wpad, const TcTile* tiles, int n_jobs, int n_splits, double* partials,
-                        int mode, int flush_every, int* err, cudaStream_t st) {
+                        int Wpad, const TcTile* tiles, int n_jobs, int panels, int n_splits,
+                        uint32_t* range, bool have_range, double* partials, int mode, int flush_every, int* err, cudaStream_t st) {
   if (mode != LEMC_GRAM_BF16X3 && mode != LEMC_GRAM_BF16X4 && mode != LEMC_GRAM_TF32X3)
     return LEMC_ERR_ARG;
   if (ldv % 64 != 0 || ldw % 64 != 0 || Wpad % 64 != 0 || n_jobs <= 0 || Wpad > ldv || Wpad > ldw)
     return LEMC_ERR_ARG;
   if (reinterpret_cast<uintptr_t>(V) % 256 != 0 || reinterpret_cast<uintptr_t>(rec_w) % 256 != 0)
     return LEMC_ERR_ARG;
-  const bool tf32 = (mode == LEMC_GRAM_TF32X3);
+  const bool half = (mode == LEMC_GRAM_TF32X3);
   TcArgs a;
   a.V = V;
   a.ldv = ldv;
@@ -791,19 +923,27 @@ int launch_gram_tc_rows(const float* V, int ldv, int total_rows, const float* re
   a.rec_w = rec_w;
   a.ldw = ldw;
   a.tiles = tiles;
+  a.range = range;
   a.partials = partials;
-  a.n_chunks_total = Wpad / (tf32 ? Cfg<true>::KC : Cfg<false>::KC);
+  a.n_chunks_total = Wpad / KC;
   a.n_splits = n_splits;
-  // The tensor core's FP32 accumulation truncates: the relative bias grows by
-  // ~4e-8 per MMA step into one accumulator, so TF32 hi/lo flushes every two
-  // K-chunks (8 steps); the BF16 split is limited by its 16-bit representation,
-  // so a longer interval costs nothing there
-  a.flush_every = flush_every > 0 ? flush_every : (tf32 ? 2 : 4);
+  // flush_every counts 32-walker chunks for TF32X3 (eight steps of two terms, as
+  // four 16-sample steps of two chunks) and K-chunks for BF16, whose 16-bit
+  // representation limits it, so a longer interval costs nothing there
+  a.flush_every = flush_every > 0 ? (half ? (flush_every > 1 ? flush_every / 2 : 1) : flush_every)
+                                  : (half ? 1 : 4);
   a.passes = (mode == LEMC_GRAM_BF16X4) ? 4 : 3;
   a.err = err;
   a.wait_cycles = g_wait_cycles;
   a.hold_loads = g_hold_loads;
-  return tf32 ? launch_t<true>(a, n_jobs, st) : launch_t<false>(a, n_jobs, st);
+  if (!have_range) {
+    if (cudaMemsetAsync(range, 0, sizeof(uint32_t) * (size_t(total_rows) + 3), st) != cudaSuccess)
+      return LEMC_ERR_CUDA;
+    row_range_kernel<<<dim3((Wpad + kRangeSpan - 1) / kRangeSpan, total_rows + 3), kRangeThreads, 0,
+                       st>>>(V, ldv, total_rows, rec_w, ldw, Wpad, range);
+  }
+  if (panels == 2) return half ? launch_t<true, 64>(a, n_jobs, st) : launch_t<false, 64>(a, n_jobs, st);
+  return half ? launch_t<true, 32>(a, n_jobs, st) : launch_t<false, 32>(a, n_jobs, st);
 }
 
 int launch_gram_tc_reduce(const double* partials, const TcTile* tiles, const TcSector* secs,
@@ -813,10 +953,6 @@ int launch_gram_tc_reduce(const double* partials, const TcTile* tiles, const TcS
   gram_tc_reduce_kernel<<<grid, 256, 0, st>>>(partials, tiles, secs, n_sec, n_tiles, n_splits,
                                               gram, plane);
   return cudaPeekAtLastError() == cudaSuccess ? LEMC_OK : LEMC_ERR_CUDA;
-}
-
-size_t gram_tc_smem_bytes(int mode) {
-  return mode == LEMC_GRAM_TF32X3 ? sizeof(Smem<true>) + 1024 : sizeof(Smem<false>) + 1024;
 }
 
 }  // namespace lemc

@@ -92,9 +92,28 @@ bool sweep_config_ok(int lanes_per_walker, int N);
 int launch_init_walkers(float2* pos, int W, int N, float radius, uint32_t seed_lo,
                         uint32_t seed_hi, cudaStream_t st);
 
+// Magnitudes for the contraction's operand scales: range[r] = FP32 bits of a bound
+// on |V[r]| over the walkers, range[rows + h] of max |W_h|, W_0 = ONE plane,
+// W_1/W_2 = ONE times the r^2/r^4 plane of rec_w; p2max[k] = range[rows + 3 + k]
+// holds the bits of max |p_k|^2.  range == nullptr: not wanted.
+struct RangeOut {
+  uint32_t* range = nullptr;
+  int rows = 0;
+  const float* rec_w = nullptr;
+  int ldw = 0;
+  uint32_t* p2max = nullptr;
+  int states = 0;
+  const uint8_t* mult = nullptr;     // [states][ldm] multiplicities of p_0..p_{ldm-1}
+  int ldm = 0;
+  const float* row_scale = nullptr;  // [states] range factors
+  const int32_t *row_re = nullptr, *row_im = nullptr;  // V rows of each state
+  float p0 = 0.f;                    // p_0 = N
+};
+
 // series_idx (may be null): the walker-mean series goes to series + 8 * *series_idx
 int launch_basis(const float2* rec_p, int W, int K, int N, const BasisProgram& prog, float* V,
-                 int ldv, double* series, const uint32_t* series_idx, cudaStream_t st);
+                 int ldv, double* series, const uint32_t* series_idx, const RangeOut& rng,
+                 cudaStream_t st);
 // Bound (cycles, 0 = default) of the contraction's mbarrier waits, and the test
 // hook that keeps its loader from issuing (so that every wait expires).
 int set_gram_wait(long long cycles, int hold_loads);
@@ -122,6 +141,7 @@ struct TcTile {
   int col0;   // first V row of the 32-row B panel
   int ksplit; // walker split index
   int slot;   // FP64 partial slot index (ksplit * n_tiles + tile)
+  int panels; // 32-row B panels to write (1 or 2: this tile's slot and the next)
 };
 // Where a sector's Gram block lives in the tile list.  A slice x = (r1 -
 // a_base) / 128 keeps B panels y = (r2 - b_base) / 32 >= 4 x only (the rest
@@ -135,12 +155,11 @@ struct TcSector {
   int a_base, b_base, n_bpanels;
 };
 int launch_gram_tc_rows(const float* V, int ldv, int total_rows, const float* rec_w, int ldw,
-                        int Wpad, const TcTile* tiles, int n_jobs, int n_splits, double* partials,
-                        int mode, int flush_every, int* err, cudaStream_t st);
+                        int Wpad, const TcTile* tiles, int n_jobs, int panels, int n_splits,
+                        uint32_t* range, bool have_range, double* partials, int mode, int flush_every, int* err, cudaStream_t st);
 int launch_gram_tc_reduce(const double* partials, const TcTile* tiles, const TcSector* secs,
                           int n_sec, int n_tiles, int n_splits, int max_dim, double* gram,
                           size_t plane, cudaStream_t st);
-size_t gram_tc_smem_bytes(int mode);
 constexpr int kTcSlot = 128 * 96;  // doubles per partial slot
 
 }  // namespace lemc
