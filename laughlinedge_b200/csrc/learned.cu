@@ -19,13 +19,14 @@
 //
 // Sampler layout: one walker per warp, positions in shared memory, lane l
 // owns particles l, l+32, ...  The 16 neighbours are found from packed
-// (distance^2, index) keys: each lane sorts its 8 keys once, then 16 rounds
-// of a warp-wide minimum (redux.sync) of the lane heads pop them in ascending
-// order; lane n keeps the n-th neighbour and forms its frame coordinates,
-// which reach every lane by shuffles.  Each lane evaluates two of the 64
-// hidden units of each layer with packed FP32x2 arithmetic; the mean phi features reach all lanes through a
-// per-warp shared-memory buffer; every reduction is an xor butterfly, so all
-// lanes hold bitwise identical values and take the same accept decision.
+// (distance^2, index) keys: each lane sorts its ceil(N/32) keys once, then 16
+// rounds of a warp-wide minimum (redux.sync) of the lane heads pop them in
+// ascending order; lane n keeps the n-th neighbour and forms its frame
+// coordinates, which reach every lane through a per-warp shared-memory buffer.
+// Each lane evaluates two of the 64 hidden units of each layer with packed FP32x2
+// arithmetic; the mean phi features go through the same buffer; every reduction is
+// an xor butterfly, so all lanes hold bitwise identical values and take the same
+// accept decision.
 // Random numbers: Philox {i, sweep, walker, 4}, drawn 32 moves at a time (one
 // move per lane) and broadcast by shuffles.
 //
@@ -39,6 +40,7 @@
 #include <cmath>
 #include <cstring>
 #include <random>
+#include <type_traits>
 #include <vector>
 
 #include "lemc_internal.h"
@@ -66,9 +68,10 @@ constexpr float kInScale = 0.5f;           // displacement feature scale (1 / 2 
 constexpr float kLogSMin = 0.f;            // log 1
 constexpr float kLogSMax = 1.386294f;      // log 4
 constexpr int kMaxN = 256;                 // packed kNN keys carry 8 index bits
-constexpr int kSlots = kMaxN / 32;         // particles per lane
+constexpr int kMaxSlots = kMaxN / 32;      // most particles per lane
 constexpr uint32_t kTagLearned = 4u, kTagTrain = 5u, kTagEs = 6u;
 constexpr int kWarpsPerBlock = 4;   // sampler / evaluation blocks
+constexpr int kSweepBlocks = 8;     // resident sweep blocks per SM
 constexpr int kTrainWarps = 16;     // ES blocks share one perturbed weight set
 constexpr float kLn2 = 0.6931471805599453f;
 
@@ -89,19 +92,34 @@ __device__ __forceinline__ int p_slot(int k) {
   return kOffW2 + ((((c & 31) * 32 + (h & 31)) << 2) | ((c >> 5) << 1) | (h >> 5));
 }
 
-// Ascending sort of a lane's 8 keys: Batcher's 19-comparator network.
-__device__ __forceinline__ void sort8(uint32_t* k) {
+// Ascending sort of a lane's S keys: comparator networks of 0, 1, 3, 5, 9, 12, 16
+// and 19 comparators (each checked against the 0-1 principle).
+template <int S>
+__device__ __forceinline__ void sort_keys(uint32_t* k) {
   auto cx = [&](int i, int j) {
     const uint32_t a = min(k[i], k[j]), b = max(k[i], k[j]);
     k[i] = a;
     k[j] = b;
   };
-  cx(0, 2); cx(1, 3); cx(4, 6); cx(5, 7);
-  cx(0, 4); cx(1, 5); cx(2, 6); cx(3, 7);
-  cx(0, 1); cx(2, 3); cx(4, 5); cx(6, 7);
-  cx(2, 4); cx(3, 5);
-  cx(1, 4); cx(3, 6);
-  cx(1, 2); cx(3, 4); cx(5, 6);
+  if constexpr (S == 2) {
+    cx(0, 1);
+  } else if constexpr (S == 3) {
+    cx(0, 2); cx(0, 1); cx(1, 2);
+  } else if constexpr (S == 4) {
+    cx(0, 2); cx(1, 3); cx(0, 1); cx(2, 3); cx(1, 2);
+  } else if constexpr (S == 5) {
+    cx(0, 3); cx(1, 4); cx(0, 2); cx(1, 3); cx(0, 1); cx(2, 4); cx(1, 2); cx(3, 4); cx(2, 3);
+  } else if constexpr (S == 6) {
+    cx(0, 5); cx(1, 3); cx(2, 4); cx(1, 2); cx(3, 4); cx(0, 3); cx(2, 5); cx(0, 1); cx(2, 3);
+    cx(4, 5); cx(1, 2); cx(3, 4);
+  } else if constexpr (S == 7) {
+    cx(0, 6); cx(2, 3); cx(4, 5); cx(0, 2); cx(1, 4); cx(3, 6); cx(0, 1); cx(2, 5); cx(3, 4);
+    cx(1, 2); cx(4, 6); cx(2, 3); cx(4, 5); cx(1, 2); cx(3, 4); cx(5, 6);
+  } else if constexpr (S == 8) {
+    cx(0, 2); cx(1, 3); cx(4, 6); cx(5, 7); cx(0, 4); cx(1, 5); cx(2, 6); cx(3, 7); cx(0, 1);
+    cx(2, 3); cx(4, 5); cx(6, 7); cx(2, 4); cx(3, 5); cx(1, 4); cx(3, 6); cx(1, 2); cx(3, 4);
+    cx(5, 6);
+  }
 }
 
 __device__ __forceinline__ float warp_sum(float v) {
@@ -110,12 +128,83 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
+// Squared distance of slot t's particle from zc, and whether the lane has one
+// there (not `self`): S = ceil(N / 32), so only the last slot can be past the end.
+template <int S>
+__device__ __forceinline__ bool slot_d2(const float2* zs, int N, int self, float2 zc, int lane, int t,
+                                        float& d2) {
+  const int j = lane + 32 * t;
+  if (!(t < S - 1 || j < N) || j == self) return false;
+  const float dx = zs[j].x - zc.x, dy = zs[j].y - zc.y;
+  d2 = fmaf(dx, dx, dy * dy);
+  return true;
+}
+__device__ __forceinline__ uint32_t pack_key(float d2, int j) {
+  return (__float_as_uint(d2) & 0xFFFFFF00u) | uint32_t(j);
+}
+
+// Keys of the lane's particles, and the products of their squared distances four
+// slots at a time (the Jastrow factors of the centre, see propose_forward).
+template <int S>
+__device__ __forceinline__ void make_keys(const float2* zs, int N, int self, float2 zc, int lane,
+                                          uint32_t* key, float* prod) {
+#pragma unroll
+  for (int t = 0; t < S; ++t) {
+    float d2;
+    key[t] = 0xFFFFFFFFu;
+    if (t % 4 == 0) prod[t / 4] = 1.f;
+    if (slot_d2<S>(zs, N, self, zc, lane, t, d2)) {
+      key[t] = pack_key(d2, lane + 32 * t);
+      prod[t / 4] *= d2;
+    }
+  }
+}
+
+// The 16 nearest in ascending key order from each lane's sorted keys: every round
+// takes the warp minimum of the lane heads and its lane pops it; lane n keeps the
+// n-th.  Depth = keys a lane can give; a shift of the whole list costs an
+// instruction per key and round, so only the first four of more are used, and
+// `lost` says (0.4 % of the time at 200 particles) that a fifth one belongs in.
+template <int Depth, int S>
+__device__ __forceinline__ uint32_t pop_nearest(uint32_t* key, int cnt, int lane, bool& lost) {
+  uint32_t mine = 0xFFFFFFFFu, m = 0u;
+#pragma unroll
+  for (int n = 0; n < kNbr; ++n) {
+    if (S > 1 || n < cnt) {  // S > 1: at least 32 other particles
+      m = __reduce_min_sync(0xffffffffu, key[0]);
+      const bool pop = key[0] == m;  // keys are unique: exactly one lane pops
+#pragma unroll
+      for (int t = 0; t < Depth - 1; ++t) key[t] = pop ? key[t + 1] : key[t];
+      key[Depth - 1] = pop ? 0xFFFFFFFFu : key[Depth - 1];
+      mine = lane == n ? m : mine;
+    }
+  }
+  lost = false;
+  if constexpr (Depth < S)
+    lost = __any_sync(0xffffffffu, key[0] == 0xFFFFFFFFu && key[Depth] < m);
+  return mine;
+}
+
+// The n-th nearest for lane n from every key of a lane: the rare case that
+// pop_nearest reports, kept out of line for the instruction cache's sake.
+template <int S>
+__device__ __noinline__ uint32_t nearest_full(const float2* zs, int N, int self, float2 zc, int lane) {
+  uint32_t key[S];
+  float prod[2];
+  bool lost;
+  make_keys<S>(zs, N, self, zc, lane, key, prod);
+  sort_keys<S>(key);
+  return pop_nearest<S, S>(key, min(kNbr, N - 1), lane, lost);
+}
+
 // The network at centre zc for particle `self` of the walker whose positions
-// are zs[0..N).  All 32 lanes call it; every lane returns the same values.
-// P holds the parameters in their shared-memory slots (p_slot); gbuf is the
-// warp's 64-float shared scratch for the mean phi features.
-__device__ NetOut net_eval(const float* __restrict__ P, const float2* zs, int N, int self,
-                           float2 zc, float invR, int lane, float* gbuf) {
+// are zs[0..N), from the lane's keys about zc.  All 32 lanes call it; every lane
+// returns the same values.  P holds the parameters in their shared-memory slots
+// (p_slot); gbuf is the warp's shared scratch of kH floats.
+template <int S>
+__device__ __forceinline__ NetOut net_eval(const float* __restrict__ P, const float2* zs, int N,
+                                           int self, float2 zc, float invR, int lane, float* gbuf,
+                                           uint32_t (&key)[S]) {
   const float r2 = zc.x * zc.x + zc.y * zc.y;
   float c = 1.f, s = 0.f;
   if (r2 > 1e-20f) {
@@ -123,56 +212,40 @@ __device__ NetOut net_eval(const float* __restrict__ P, const float2* zs, int N,
     c = zc.x * ri;
     s = zc.y * ri;
   }
-  uint32_t key[kSlots];
-#pragma unroll
-  for (int t = 0; t < kSlots; ++t) {
-    const int j = lane + 32 * t;
-    key[t] = 0xFFFFFFFFu;
-    if (j < N && j != self) {
-      const float dx = zs[j].x - zc.x, dy = zs[j].y - zc.y;
-      key[t] = (__float_as_uint(fmaf(dx, dx, dy * dy)) & 0xFFFFFF00u) | uint32_t(j);
-    }
-  }
-  // The 16 nearest in ascending key order: each lane sorts its keys once, then
-  // every round takes the warp minimum of the lane heads and its lane pops it;
-  // lane n keeps the n-th neighbour.
-  static_assert(kSlots == 8, "sort8 network");
   static_assert(kNbr <= 32, "one neighbour per lane");
-  sort8(key);
-  // every other particle has a finite key, so exactly min(16, N - 1) rounds
-  // pop a neighbour; the rounds are unrolled under that uniform bound
+  constexpr int kDepth = S > 4 ? 4 : S;
   const int cnt = min(kNbr, N - 1);
-  uint32_t mine = 0xFFFFFFFFu;
-#pragma unroll
-  for (int n = 0; n < kNbr; ++n) {
-    if (n < cnt) {
-      const uint32_t m = __reduce_min_sync(0xffffffffu, key[0]);
-      const bool pop = key[0] == m;  // keys are unique: exactly one lane pops
-#pragma unroll
-      for (int t = 0; t < kSlots - 1; ++t) key[t] = pop ? key[t + 1] : key[t];
-      key[kSlots - 1] = pop ? 0xFFFFFFFFu : key[kSlots - 1];
-      mine = lane == n ? m : mine;
-    }
+  sort_keys<S>(key);
+  bool lost;
+  uint32_t mine = pop_nearest<kDepth, S>(key, cnt, lane, lost);
+  if constexpr (kDepth < S) {
+    if (lost) mine = nearest_full<S>(zs, N, self, zc, lane);  // warp-uniform
   }
   // each lane forms the frame coordinates of its own neighbour once; phi then
-  // runs over the neighbours in the same ascending order, their coordinates
-  // broadcast by shuffles, two hidden units per lane as one packed pair
-  float xr = 0.f, xt = 0.f;
+  // runs over the neighbours in the same ascending order, two hidden units per lane
+  // as one packed pair
+  float2* nb = reinterpret_cast<float2*>(gbuf);
   if (lane < cnt) {
     const int j = int(mine & 0xFFu);
     const float dx = zs[j].x - zc.x, dy = zs[j].y - zc.y;
-    xr = (dx * c + dy * s) * kInScale;
-    xt = (dy * c - dx * s) * kInScale;
+    const float xr = (dx * c + dy * s) * kInScale;
+    const float xt = (dy * c - dx * s) * kInScale;
+    nb[lane] = make_float2(xr, xt);
   }
+  __syncwarp();
   const float2 W0X = make_float2(P[kOffW1 + 2 * lane], P[kOffW1 + 2 * (lane + 32)]);
   const float2 W0Y = make_float2(P[kOffW1 + 2 * lane + 1], P[kOffW1 + 2 * (lane + 32) + 1]);
   const float2 B0 = make_float2(P[kOffB1 + lane], P[kOffB1 + lane + 32]);
   float2 g = make_float2(0.f, 0.f);
 #pragma unroll
-  for (int n = 0; n < kNbr; ++n) {
-    if (n < cnt) {
-      const float a = __shfl_sync(0xffffffffu, xr, n), b = __shfl_sync(0xffffffffu, xt, n);
-      const float2 h = __ffma2_rn(W0X, make_float2(a, a), __ffma2_rn(W0Y, make_float2(b, b), B0));
+  for (int n = 0; n < kNbr; n += 2) {
+    const float4 x = reinterpret_cast<const float4*>(nb)[n / 2];
+    if (S > 1 || n < cnt) {
+      const float2 h = __ffma2_rn(W0X, make_float2(x.x, x.x), __ffma2_rn(W0Y, make_float2(x.y, x.y), B0));
+      g = __fadd2_rn(g, make_float2(fmaxf(h.x, 0.f), fmaxf(h.y, 0.f)));
+    }
+    if (S > 1 || n + 1 < cnt) {
+      const float2 h = __ffma2_rn(W0X, make_float2(x.z, x.z), __ffma2_rn(W0Y, make_float2(x.w, x.w), B0));
       g = __fadd2_rn(g, make_float2(fmaxf(h.x, 0.f), fmaxf(h.y, 0.f)));
     }
   }
@@ -196,7 +269,7 @@ __device__ NetOut net_eval(const float* __restrict__ P, const float2* zs, int N,
     kk = __ffma2_rn(make_float2(w.z, w.w), make_float2(gb, gb), kk);
     kk = __ffma2_rn(make_float2(w.x, w.y), make_float2(ga, ga), kk);
   };
-#pragma unroll 2
+#pragma unroll
   for (int v4 = 0; v4 < 8; ++v4) {
     const float4 ga = G4[v4], gb = G4[8 + v4];
     rho_in(4 * v4, ga.x, gb.x);
@@ -204,9 +277,7 @@ __device__ NetOut net_eval(const float* __restrict__ P, const float2* zs, int N,
     rho_in(4 * v4 + 2, ga.z, gb.z);
     rho_in(4 * v4 + 3, ga.w, gb.w);
   }
-  float k0 = kk.x, k1 = kk.y;
-  k0 = fmaxf(k0, 0.f);
-  k1 = fmaxf(k1, 0.f);
+  const float k0 = fmaxf(kk.x, 0.f), k1 = fmaxf(kk.y, 0.f);
   float o[4];
 #pragma unroll
   for (int q = 0; q < 4; ++q)
@@ -237,11 +308,12 @@ struct Forward {
 // ln A = part + ln q(z | z') never exceeds part + kLogQbMax in FP32 either.
 constexpr float kLogQbMax = -2.f * kLogSMin;
 
-__device__ Forward propose_forward(const float* __restrict__ P, const float2* zs, int N, int i,
-                                   float invR, float m, float e_r, float e_t, int lane,
-                                   float* gbuf) {
-  const float2 zo = zs[i];
-  const NetOut f = net_eval(P, zs, N, i, zo, invR, lane, gbuf);
+// key: out, the lane's keys about the proposed position; po: the products of the
+// squared distances from z, formed with the keys about it
+template <int S>
+__device__ __forceinline__ Forward propose_forward(const NetOut& f, const float2* zs, int N, int i,
+                                                   float2 zo, const float (&po)[2], float m, float e_r,
+                                                   float e_t, int lane, uint32_t (&key)[S]) {
   const float sr = __expf(f.lr), st = __expf(f.lt);
   const float dr = fmaf(sr, e_r, f.mr), dt = fmaf(st, e_t, f.mt);
   const float r2 = zo.x * zo.x + zo.y * zo.y;
@@ -256,23 +328,13 @@ __device__ Forward propose_forward(const float* __restrict__ P, const float2* zs
   const float log_qf = -0.5f * (e_r * e_r + e_t * e_t) - f.lr - f.lt;
   // target ratio: m sum_j ln(|z'-z_j|^2 / |z-z_j|^2) - (|z'|^2 - |z|^2) / 2
   // FP32 products of four squared distances, one log2 per product: for
-  // distances between 1e-4 and 1e4 a product stays within 1e-32 .. 1e32
+  // distances between 1e-4 and 1e4 a product stays within 1e-32 .. 1e32.
+  // The distances from z' give the keys that the reverse network will need.
   float lj = 0.f;
+  float pn[2];
+  make_keys<S>(zs, N, i, fw.zn, lane, key, pn);
 #pragma unroll
-  for (int t0 = 0; t0 < kSlots; t0 += 4) {
-    float pn = 1.f, po = 1.f;
-#pragma unroll
-    for (int t = t0; t < t0 + 4; ++t) {
-      const int j = lane + 32 * t;
-      if (j < N && j != i) {
-        const float2 zj = zs[j];
-        const float ax = fw.zn.x - zj.x, ay = fw.zn.y - zj.y, ox = zo.x - zj.x, oy = zo.y - zj.y;
-        pn *= fmaf(ax, ax, ay * ay);
-        po *= fmaf(ox, ox, oy * oy);
-      }
-    }
-    lj += __log2f(pn) - __log2f(po);
-  }
+  for (int q = 0; q < (S + 3) / 4; ++q) lj += __log2f(pn[q]) - __log2f(po[q]);
   lj = warp_sum(lj);
   const float rn2 = fw.zn.x * fw.zn.x + fw.zn.y * fw.zn.y;
   const float dlp = m * kLn2 * lj - 0.5f * (rn2 - r2);
@@ -281,11 +343,8 @@ __device__ Forward propose_forward(const float* __restrict__ P, const float2* zs
   return fw;
 }
 
-// ln q(z_i | z'): the network at the proposed configuration (particle i at zn).
-__device__ float reverse_log_density(const float* __restrict__ P, const float2* zs, int N, int i,
-                                     float2 zn, float invR, int lane, float* gbuf) {
-  const float2 zo = zs[i];
-  const NetOut b = net_eval(P, zs, N, i, zn, invR, lane, gbuf);
+// ln q(z_i | z') from the network b at the proposed configuration (particle i at zn).
+__device__ __forceinline__ float reverse_log_density(const NetOut& b, float2 zo, float2 zn) {
   const float rn2 = zn.x * zn.x + zn.y * zn.y;
   float cb = 1.f, sb = 0.f;
   if (rn2 > 1e-20f) {
@@ -299,12 +358,44 @@ __device__ float reverse_log_density(const float* __restrict__ P, const float2* 
   return -0.5f * (ur * ur + ut * ut) - b.lr - b.lt;
 }
 
-__device__ Move propose(const float* __restrict__ P, const float2* zs, int N, int i, float invR,
-                        float m, float e_r, float e_t, int lane, float* gbuf) {
-  const Forward fw = propose_forward(P, zs, N, i, invR, m, e_r, e_t, lane, gbuf);
+// One proposed move of particle i: the network at z, the move, and, where `wanted`
+// says so, the network at the proposed configuration; lq is ln q(z | z') then, and
+// the result whether it was formed.  Both networks run through one copy of the code
+// (a rolled loop), which leaves the instruction cache room for its loops unrolled:
+// a copy each took 73.0 ms for four sweeps at N=200, W=65536, this 72.0.
+template <int S, class Wanted>
+__device__ __forceinline__ bool move_step(const float* __restrict__ P, const float2* zs, int N, int i,
+                                          float invR, float m, float e_r, float e_t, int lane,
+                                          float* gbuf, Forward& fw, float& lq, Wanted&& wanted) {
+  const float2 zo = zs[i];
+  float2 zc = zo;
+  float po[2];
+  uint32_t key[S];
+  make_keys<S>(zs, N, i, zo, lane, key, po);
+#pragma unroll 1
+  for (int pass = 0; pass < 2; ++pass) {
+    const NetOut net = net_eval<S>(P, zs, N, i, zc, invR, lane, gbuf, key);
+    if (pass == 0) {
+      fw = propose_forward<S>(net, zs, N, i, zo, po, m, e_r, e_t, lane, key);
+      zc = fw.zn;
+      if (!wanted(fw)) return false;
+    } else {
+      lq = reverse_log_density(net, zo, zc);
+    }
+  }
+  return true;
+}
+
+template <int S>
+__device__ __forceinline__ Move propose(const float* __restrict__ P, const float2* zs, int N, int i,
+                                        float invR, float m, float e_r, float e_t, int lane,
+                                        float* gbuf) {
+  Forward fw;
+  float lq = 0.f;
+  move_step<S>(P, zs, N, i, invR, m, e_r, e_t, lane, gbuf, fw, lq, [](const Forward&) { return true; });
   Move mv;
   mv.zn = fw.zn;
-  mv.log_a = fw.part + reverse_log_density(P, zs, N, i, fw.zn, invR, lane, gbuf);
+  mv.log_a = fw.part + lq;
   mv.jump2 = fw.jump2;
   return mv;
 }
@@ -321,61 +412,9 @@ __device__ void load_params(float* P, const __nv_bfloat16* w) {
   for (int k = threadIdx.x; k < kNParams; k += blockDim.x) P[p_slot(k)] = __bfloat162float(w[k]);
 }
 
-__global__ void __launch_bounds__(kWarpsPerBlock * 32)
-learned_sweep_kernel(const SweepArgs a, const __nv_bfloat16* __restrict__ wts) {
-  __shared__ __align__(16) float P[kNParams];
-  __shared__ __align__(16) float gsm[kWarpsPerBlock][kH];
-  extern __shared__ float2 zsm[];
-  load_params(P, wts);
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const int w = blockIdx.x * kWarpsPerBlock + wib;
-  const bool live = w < a.W;
+// One walker's record from its positions, by one warp.
+__device__ void learned_record(const SweepArgs& a, const float2* zs, int w, int lane) {
   const int N = a.N;
-  float2* zs = zsm + size_t(wib) * N;
-  if (live)
-    for (int j = lane; j < N; j += 32) zs[j] = a.pos[size_t(w) * N + j];
-  __syncthreads();
-  if (!live) return;
-  __syncwarp();
-  const uint32_t sweep_base = a.sweep0 + (a.sweep_ctr ? *a.sweep_ctr : 0u);
-  const float m = float(a.m);
-  uint32_t nacc = 0, nrev = 0;
-  for (int sw = 0; sw < a.n_sweeps; ++sw) {
-    const uint32_t sweep = sweep_base + uint32_t(sw);
-    float er_l = 0.f, et_l = 0.f, lu_l = 0.f;
-    for (int i = 0; i < N; ++i) {
-      // the randoms of move i come from Philox {i, sweep, walker, 4}: lane l
-      // draws those of move 32 b + l for the whole block b of 32 moves
-      if ((i & 31) == 0) {
-        const U4 r = philox4x32_10(U4{uint32_t(i + lane), sweep, uint32_t(w), kTagLearned},
-                                   a.seed_lo, a.seed_hi);
-        box_muller(r.x, r.y, er_l, et_l);
-        lu_l = __logf(u01(r.z));
-      }
-      const float er = __shfl_sync(0xffffffffu, er_l, i & 31);
-      const float et = __shfl_sync(0xffffffffu, et_l, i & 31);
-      const float lu = __shfl_sync(0xffffffffu, lu_l, i & 31);
-      // the reverse density is only evaluated when it can change the decision:
-      // if ln u >= part + kLogQbMax, ln u >= ln A in FP32 and the move is
-      // rejected as the full ratio would reject it (warp-uniform test)
-      const Forward fw = propose_forward(P, zs, N, i, a.invR, m, er, et, lane, gsm[wib]);
-      bool acc = false;
-      if (lu < fw.part + kLogQbMax) {
-        acc = lu < fw.part + reverse_log_density(P, zs, N, i, fw.zn, a.invR, lane, gsm[wib]);
-        ++nrev;
-      }
-      __syncwarp();
-      if (acc) {
-        if (lane == (i & 31)) zs[i] = fw.zn;
-        ++nacc;
-      }
-      __syncwarp();
-    }
-  }
-  for (int j = lane; j < N; j += 32) a.pos[size_t(w) * N + j] = zs[j];
-  if (a.accepted && lane == 0) a.accepted[w] += nacc;
-  if (a.reverse_evals && lane == 0) a.reverse_evals[w] += nrev;
-  if (!a.measure) return;
   // measurement record, the plain sweep's layout: four degrees per pass over
   // the particles (w^k by the same sequence of multiplications in every pass),
   // then r^2 / r^4, then one pass per probe, so that few registers are live
@@ -443,8 +482,76 @@ learned_sweep_kernel(const SweepArgs a, const __nv_bfloat16* __restrict__ wts) {
   }
 }
 
+// What bounds the sweep: shared-memory bandwidth (353 wavefronts a move, 81 % of the
+// peak, half of them the W2 records) with 1220 instructions a move at 72 % of the
+// issue slots.  Measured (B200, N=200, W=65536): 21.5 -> 18.0 ms a sweep, from 1492
+// instructions: slots compiled for ceil(N/32), four keys a lane in the 16 rounds,
+// the distances of the Jastrow factors shared with the searches, neighbour
+// coordinates read back two at a time.  Two walkers a warp, which reads W2 once for
+// both (264 wavefronts), took 19.1 ms: 96 registers leave 20 warps.
+template <int S>
+__global__ void __launch_bounds__(kWarpsPerBlock * 32, kSweepBlocks)
+learned_sweep_kernel(const SweepArgs a, const __nv_bfloat16* __restrict__ wts) {
+  __shared__ __align__(16) float P[kNParams];
+  __shared__ __align__(16) float gsm[kWarpsPerBlock][kH];
+  extern __shared__ float2 zsm[];
+  load_params(P, wts);
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const int w = blockIdx.x * kWarpsPerBlock + wib;
+  const bool live = w < a.W;
+  const int N = a.N;
+  float2* zs = zsm + size_t(wib) * N;
+  if (live)
+    for (int j = lane; j < N; j += 32) zs[j] = a.pos[size_t(w) * N + j];
+  __syncthreads();
+  if (!live) return;
+  __syncwarp();
+  const uint32_t sweep_base = a.sweep0 + (a.sweep_ctr ? *a.sweep_ctr : 0u);
+  const float m = float(a.m);
+  uint32_t nacc = 0, nrev = 0;
+  for (int sw = 0; sw < a.n_sweeps; ++sw) {
+    const uint32_t sweep = sweep_base + uint32_t(sw);
+    float er_l = 0.f, et_l = 0.f, lu_l = 0.f;
+    for (int i = 0; i < N; ++i) {
+      // the randoms of move i come from Philox {i, sweep, walker, 4}: lane l
+      // draws those of move 32 b + l for the whole block b of 32 moves
+      if ((i & 31) == 0) {
+        const U4 r = philox4x32_10(U4{uint32_t(i + lane), sweep, uint32_t(w), kTagLearned},
+                                   a.seed_lo, a.seed_hi);
+        box_muller(r.x, r.y, er_l, et_l);
+        lu_l = __logf(u01(r.z));
+      }
+      const float er = __shfl_sync(0xffffffffu, er_l, i & 31);
+      const float et = __shfl_sync(0xffffffffu, et_l, i & 31);
+      const float lu = __shfl_sync(0xffffffffu, lu_l, i & 31);
+      // the reverse density is only evaluated when it can change the decision:
+      // if ln u >= part + kLogQbMax, ln u >= ln A in FP32 and the move is
+      // rejected as the full ratio would reject it (warp-uniform test)
+      Forward fw;
+      float lq = 0.f;
+      bool acc = false;
+      if (move_step<S>(P, zs, N, i, a.invR, m, er, et, lane, gsm[wib], fw, lq,
+                       [&](const Forward& f) { return lu < f.part + kLogQbMax; })) {
+        acc = lu < fw.part + lq;
+        ++nrev;
+      }
+      __syncwarp();
+      if (acc) {
+        if (lane == (i & 31)) zs[i] = fw.zn;
+        ++nacc;
+      }
+      __syncwarp();
+    }
+  }
+  for (int j = lane; j < N; j += 32) a.pos[size_t(w) * N + j] = zs[j];
+  if (a.accepted && lane == 0) a.accepted[w] += nacc;
+  if (a.reverse_evals && lane == 0) a.reverse_evals[w] += nrev;
+  if (a.measure) learned_record(a, zs, w, lane);
+}
+
 // Network outputs and proposal densities for given (configuration, particle,
 // eps): out[s] = {mu_r, mu_t, log s_r, log s_t, z'.x, z'.y, ln A, |z'-z|^2}.
+template <int S>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 learned_eval_kernel(const float2* __restrict__ cfgs, int n, int N, float invR, float m,
                     const int32_t* __restrict__ particle, const float* __restrict__ eps,
@@ -462,8 +569,11 @@ learned_eval_kernel(const float2* __restrict__ cfgs, int n, int N, float invR, f
   if (sidx >= n) return;
   __syncwarp();
   const int i = particle[sidx];
-  const NetOut f = net_eval(P, zs, N, i, zs[i], invR, lane, gsm[wib]);
-  const Move mv = propose(P, zs, N, i, invR, m, eps[2 * sidx], eps[2 * sidx + 1], lane, gsm[wib]);
+  uint32_t key[S];
+  float po[2];
+  make_keys<S>(zs, N, i, zs[i], lane, key, po);
+  const NetOut f = net_eval<S>(P, zs, N, i, zs[i], invR, lane, gsm[wib], key);
+  const Move mv = propose<S>(P, zs, N, i, invR, m, eps[2 * sidx], eps[2 * sidx + 1], lane, gsm[wib]);
   if (lane == 0) {
     float* o = out + size_t(sidx) * 8;
     o[0] = f.mr;
@@ -479,6 +589,7 @@ learned_eval_kernel(const float2* __restrict__ cfgs, int n, int N, float invR, f
 
 // ES objective: block (x, pert) evaluates kWarpsPerBlock samples with the
 // parameters theta + sign * sigma * e_pair; J[pert] += sum of min(1, A) |dz|^2.
+template <int S>
 __global__ void __launch_bounds__(kTrainWarps * 32)
 es_objective_kernel(const float2* __restrict__ cfgs, int n_cfg, int N, float invR, float m,
                     const float* __restrict__ theta, float es_sigma, uint32_t step, uint32_t k0,
@@ -509,7 +620,7 @@ es_objective_kernel(const float2* __restrict__ cfgs, int n_cfg, int N, float inv
   if (live) {
     float er, et;
     box_muller(r.z, r.w, er, et);
-    const Move mv = propose(P, zs, N, i, invR, m, er, et, lane, gsm[wib]);
+    const Move mv = propose<S>(P, zs, N, i, invR, m, er, et, lane, gsm[wib]);
     val = (mv.log_a >= 0.f ? 1.f : __expf(mv.log_a)) * mv.jump2;
     if (!(val == val)) val = 0.f;
   }
@@ -561,6 +672,23 @@ __global__ void to_bf16_kernel(const float* __restrict__ theta, __nv_bfloat16* _
   if (k < kNParams) wts[k] = __float2bfloat16_rn(theta[k]);
 }
 
+// f(integral constant S) for the S = ceil(N / 32) particle slots per lane that the
+// kernels are compiled for (N <= kMaxN)
+template <class F>
+void with_slots(int N, F&& f) {
+  static_assert(kMaxSlots == 8, "one case per slot count");
+  switch ((N + 31) / 32) {
+    case 1: f(std::integral_constant<int, 1>{}); break;
+    case 2: f(std::integral_constant<int, 2>{}); break;
+    case 3: f(std::integral_constant<int, 3>{}); break;
+    case 4: f(std::integral_constant<int, 4>{}); break;
+    case 5: f(std::integral_constant<int, 5>{}); break;
+    case 6: f(std::integral_constant<int, 6>{}); break;
+    case 7: f(std::integral_constant<int, 7>{}); break;
+    default: f(std::integral_constant<int, 8>{}); break;
+  }
+}
+
 size_t walker_smem(int N, int warps = kWarpsPerBlock) { return size_t(warps) * N * sizeof(float2); }
 
 }  // namespace
@@ -568,8 +696,10 @@ size_t walker_smem(int N, int warps = kWarpsPerBlock) { return size_t(warps) * N
 int launch_learned_sweep(const SweepArgs& a, const void* wts, cudaStream_t st) {
   if (a.N > kMaxN || a.K > kMaxDegree) return LEMC_ERR_CAPACITY;
   const int blocks = (a.W + kWarpsPerBlock - 1) / kWarpsPerBlock;
-  learned_sweep_kernel<<<blocks, kWarpsPerBlock * 32, walker_smem(a.N), st>>>(
-      a, static_cast<const __nv_bfloat16*>(wts));
+  with_slots(a.N, [&](auto s) {
+    learned_sweep_kernel<s.value><<<blocks, kWarpsPerBlock * 32, walker_smem(a.N), st>>>(
+        a, static_cast<const __nv_bfloat16*>(wts));
+  });
   return cudaPeekAtLastError() == cudaSuccess ? LEMC_OK : LEMC_ERR_CUDA;
 }
 
@@ -700,9 +830,11 @@ extern "C" int lemc_proposal_eval(const lemc_proposal* p, const float* host_xy, 
     ok(cudaMemcpy(d_e, eps, sizeof(float) * 2 * n, cudaMemcpyHostToDevice));
   }
   if (st == LEMC_OK) {
-    learned_eval_kernel<<<(n + kWarpsPerBlock - 1) / kWarpsPerBlock, kWarpsPerBlock * 32,
-                          walker_smem(N)>>>(d_cfg, n, N, p->invR, float(p->m), d_i, d_e, p->wts,
-                                            d_o);
+    with_slots(N, [&](auto s) {
+      learned_eval_kernel<s.value><<<(n + kWarpsPerBlock - 1) / kWarpsPerBlock, kWarpsPerBlock * 32,
+                                     walker_smem(N)>>>(d_cfg, n, N, p->invR, float(p->m), d_i, d_e,
+                                                       p->wts, d_o);
+    });
     ok(cudaPeekAtLastError());
     ok(cudaDeviceSynchronize());
     ok(cudaMemcpy(out, d_o, sizeof(float) * 8 * n, cudaMemcpyDeviceToHost));
@@ -724,10 +856,14 @@ extern "C" int lemc_proposal_train(lemc_proposal* p, const void* configs, int n_
   const size_t smem_static = sizeof(float) * (kNParams + kTrainWarps * kH + kTrainWarps);
   const size_t smem_dyn = walker_smem(N, kTrainWarps);
   if (smem_static + smem_dyn > 227 * 1024) return LEMC_ERR_CAPACITY;
-  if (smem_static + smem_dyn > 48 * 1024 &&
-      cudaFuncSetAttribute(es_objective_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           int(smem_dyn)) != cudaSuccess)
-    return LEMC_ERR_CUDA;
+  if (smem_static + smem_dyn > 48 * 1024) {
+    cudaError_t e = cudaSuccess;
+    with_slots(N, [&](auto s) {
+      e = cudaFuncSetAttribute(es_objective_kernel<s.value>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               int(smem_dyn));
+    });
+    if (e != cudaSuccess) return LEMC_ERR_CUDA;
+  }
   if (p->J_cap < 2 * tc->pairs) {
     cudaFree(p->J);
     p->J = nullptr;
@@ -745,9 +881,11 @@ extern "C" int lemc_proposal_train(lemc_proposal* p, const void* configs, int n_
   for (int s = 0; s < tc->steps; ++s) {
     const uint32_t step = uint32_t(p->train_steps);
     if (cudaMemsetAsync(p->J, 0, sizeof(double) * 2 * tc->pairs) != cudaSuccess) return LEMC_ERR_CUDA;
-    es_objective_kernel<<<grid, kTrainWarps * 32, walker_smem(N, kTrainWarps)>>>(
-        static_cast<const float2*>(configs), n_cfg, N, p->invR, float(p->m), p->theta,
-        tc->es_sigma, step, k0, k1, tc->batch, p->J);
+    with_slots(N, [&](auto sl) {
+      es_objective_kernel<sl.value><<<grid, kTrainWarps * 32, walker_smem(N, kTrainWarps)>>>(
+          static_cast<const float2*>(configs), n_cfg, N, p->invR, float(p->m), p->theta, tc->es_sigma,
+          step, k0, k1, tc->batch, p->J);
+    });
     es_adam_kernel<<<(kNParams + 255) / 256, 256>>>(p->theta, p->am, p->av, p->wts, p->J,
                                                     tc->pairs, tc->batch, tc->es_sigma, tc->lr,
                                                     step, k0, k1, p->trace + s);
