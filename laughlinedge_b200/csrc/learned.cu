@@ -412,8 +412,15 @@ __device__ void load_params(float* P, const __nv_bfloat16* w) {
   for (int k = threadIdx.x; k < kNParams; k += blockDim.x) P[p_slot(k)] = __bfloat162float(w[k]);
 }
 
+// w^k -> w^{k+1}, with the fused products spelt out (as in the powers skipped
+// below): the recorded power sums then do not depend on how the compiler contracts
+// them in its context.
+__device__ __forceinline__ float2 next_power(float2 pw, float2 w) {
+  return make_float2(fmaf(pw.x, w.x, -__fmul_rn(pw.y, w.y)), fmaf(pw.y, w.x, __fmul_rn(pw.x, w.y)));
+}
+
 // One walker's record from its positions, by one warp.
-__device__ void learned_record(const SweepArgs& a, const float2* zs, int w, int lane) {
+__device__ __forceinline__ void learned_record(const SweepArgs& a, const float2* zs, int w, int lane) {
   const int N = a.N;
   // measurement record, the plain sweep's layout: four degrees per pass over
   // the particles (w^k by the same sequence of multiplications in every pass),
@@ -428,12 +435,13 @@ __device__ void learned_record(const SweepArgs& a, const float2* zs, int w, int 
       const float2 wv = make_float2(z.x * a.invR, z.y * a.invR);
       float2 pw = wv;
       for (int k = 0; k < k0; ++k)
-        pw = make_float2(pw.x * wv.x - pw.y * wv.y, pw.x * wv.y + pw.y * wv.x);
+        pw = make_float2(fmaf(pw.x, wv.x, -__fmul_rn(pw.y, wv.y)),
+                         fmaf(pw.x, wv.y, __fmul_rn(pw.y, wv.x)));
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         acc[k].x += pw.x;
         acc[k].y += pw.y;
-        pw = make_float2(pw.x * wv.x - pw.y * wv.y, pw.x * wv.y + pw.y * wv.x);
+        pw = next_power(pw, wv);
       }
     }
 #pragma unroll
