@@ -218,10 +218,7 @@ struct lemc_ctx {
   DevBuf<double> tc_partials;
   int tc_splits = 1;
   bool tc_dirty = false;  // the partial slots hold sums not yet folded into `gram`
-  // read-back of a block: unscaled planes with their status on the device, and
-  // pinned host memory they pass through
-  DevBuf<double> d_read;
-  double* h_read = nullptr;
+  DevBuf<double> d_read;  // read-back of a block: its unscaled planes with their status
   DevBuf<double> d_row_scale64;  // per basis row
 
   bool walkers_ready = false;
@@ -724,15 +721,14 @@ __global__ void read_block_kernel(const double2* __restrict__ src, size_t plane,
   if (blockIdx.x == 0 && threadIdx.x == 0 && *err != 0) atomicOr(head, 2ull);
 }
 
-// Copies the block to the caller's buffers.  The planes leave the device in one
-// piece through pinned memory, half a buffer landing while the other is handed on.
-// A copy per plane into pageable memory, a fold of every partial slot before each
-// sector and the factors undone in a host loop took 8.7 + 3.0 + some 10 ms for the
-// 20 sectors of the 2713-state basis; the copies now take 0.9 ms and the whole call
-// of eight sweeps went from 95 to 79 ms, most of the rest of the read-back being
-// the page faults of the caller's fresh buffers.
-constexpr size_t kReadHalf = size_t(1) << 19;   // doubles: two 4 MB halves
-constexpr size_t kReadSmall = size_t(1) << 13;
+// Copies the block to the caller's buffers: one piece through a local buffer when it
+// is small, else a copy per plane.  A fold of every partial slot before each sector,
+// its planes one by one with the factors undone in a host loop took 12 ms on the
+// device and some 10 ms on the host for the 20 sectors of the 2713-state basis; now
+// now.  Pinned staging would not pay: getting the memory costs 3 to 13 ms
+// whatever its size, and what remains of a copy is mostly the page faults of the
+// caller's fresh buffers (5 GB/s; 15 GB/s into touched pages).
+constexpr size_t kReadSmall = size_t(1) << 13;  // doubles
 int read_block(lemc_ctx* c, const double* src, size_t plane, int da, int db, const double* sa,
                const double* sb, double* const (&outs)[3], bool* finite) {
   const size_t n = 2 * size_t(da) * db;  // doubles of a plane
@@ -741,39 +737,25 @@ int read_block(lemc_ctx* c, const double* src, size_t plane, int da, int db, con
     if (outs[h]) idx[np++] = h;
   const size_t total = 2 * kReadHead + np * n;
   LEMC_TRY(c->d_read.alloc(total));
-  // a small block is not worth pinned memory (0.1 ms and more to get)
-  std::vector<double> small(total <= kReadSmall ? total : 0);
-  if (total > kReadSmall && !c->h_read)
-    LEMC_CUDA(cudaMallocHost(&c->h_read, 2 * kReadHalf * sizeof(double)));
   LEMC_CUDA(cudaMemsetAsync(c->d_read.p, 0, 2 * kReadHead * sizeof(double), c->stream));
   const size_t blocks = std::min<size_t>((size_t(da) * db + 255) / 256, 148 * 8);
   read_block_kernel<<<unsigned(blocks), 256, 0, c->stream>>>(
       reinterpret_cast<const double2*>(src), plane, da, db, sa, sb, np, make_int3(idx[0], idx[1], idx[2]),
       c->err.p, c->d_read.p);
   LEMC_CUDA(cudaPeekAtLastError());
-  auto start = [&](size_t k) {  // piece k of kReadHalf doubles into half k % 2
-    const size_t b = k * kReadHalf, len = std::min(kReadHalf, total - b);
-    double* to = small.empty() ? c->h_read + (k & 1) * kReadHalf : small.data();
-    LEMC_CUDA(cudaMemcpyAsync(to, c->d_read.p + b, len * sizeof(double),
-                              cudaMemcpyDeviceToHost, c->stream));
-    LEMC_CUDA(cudaEventRecord(c->ev[k & 1], c->stream));
-    return int(LEMC_OK);
-  };
-  const size_t pieces = (total + kReadHalf - 1) / kReadHalf;
-  LEMC_TRY(start(0));
+  std::vector<double> host(total <= kReadSmall ? total : 2 * kReadHead);
+  LEMC_CUDA(cudaMemcpyAsync(host.data(), c->d_read.p, host.size() * sizeof(double),
+                            cudaMemcpyDeviceToHost, c->stream));
+  if (total > kReadSmall)
+    for (int h = 0; h < np; ++h)
+      LEMC_CUDA(cudaMemcpyAsync(outs[idx[h]], c->d_read.p + 2 * kReadHead + h * n, n * sizeof(double),
+                                cudaMemcpyDeviceToHost, c->stream));
+  LEMC_CUDA(cudaStreamSynchronize(c->stream));
+  if (total <= kReadSmall)
+    for (int h = 0; h < np; ++h)
+      std::memcpy(outs[idx[h]], host.data() + 2 * kReadHead + h * n, n * sizeof(double));
   unsigned long long head = 0;
-  for (size_t k = 0; k < pieces; ++k) {
-    if (k + 1 < pieces) LEMC_TRY(start(k + 1));
-    LEMC_CUDA(cudaEventSynchronize(c->ev[k & 1]));
-    const double* piece = small.empty() ? c->h_read + (k & 1) * kReadHalf : small.data();
-    if (k == 0) std::memcpy(&head, piece, sizeof(head));
-    // the parts of the planes that this piece holds
-    const size_t b = k * kReadHalf, e = std::min(total, b + kReadHalf);
-    for (int h = 0; h < np; ++h) {
-      const size_t p0 = 2 * kReadHead + h * n, lo = std::max(b, p0), hi = std::min(e, p0 + n);
-      if (lo < hi) std::memcpy(outs[idx[h]] + (lo - p0), piece + (lo - b), (hi - lo) * sizeof(double));
-    }
-  }
+  std::memcpy(&head, host.data(), sizeof(head));
   *finite = (head & 1) == 0;
   return (head & 2) ? LEMC_ERR_TIMEOUT : LEMC_OK;
 }
@@ -917,7 +899,6 @@ int lemc_destroy(lemc_ctx* c) {
   c->d_row_mult.release();
   c->d_row_scale64.release();
   c->d_read.release();
-  if (c->h_read) cudaFreeHost(c->h_read);
   for (auto& e : c->ev)
     if (e) cudaEventDestroy(e);
   for (auto& e : c->pev) cudaEventDestroy(e);

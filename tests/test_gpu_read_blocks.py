@@ -1,4 +1,4 @@
-"""Read-back of Gram and cross blocks around the sizes of its staging pieces, with
+"""Read-back of Gram and cross blocks, small (one piece) and large (plane by plane), with
 planes left out, after reset and repeated, against the same sums in numpy."""
 import ctypes as C
 
@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("mode", [0, 3])
 def test_read_blocks(lemc, cuda_ctx, mode):
     torch, lib = cuda_ctx, lemc.load()
-    # 1, 77 and 490 states: pageable, 35 k and 1.4 M doubles (two more pieces than halves)
+    # 1, 77 and 490 states: 8, 35 k and 1.4 M doubles
     sectors, W = [0, 12, 19], 64
     g = np.random.default_rng(1)
     smp = lemc.Sampler(lemc.SamplerConfig(20, 3, W, gram_mode=mode), sectors, probes=[7])
