@@ -725,7 +725,7 @@ __global__ void read_block_kernel(const double2* __restrict__ src, size_t plane,
 // is small, else a copy per plane.  A fold of every partial slot before each sector,
 // its planes one by one with the factors undone in a host loop took 12 ms on the
 // device and some 10 ms on the host for the 20 sectors of the 2713-state basis; now
-// now.  Pinned staging would not pay: getting the memory costs 3 to 13 ms
+// 0.3 ms and the copies.  Pinned staging would not pay: getting the memory costs 3 to 13 ms
 // whatever its size, and what remains of a copy is mostly the page faults of the
 // caller's fresh buffers (5 GB/s; 15 GB/s into touched pages).
 constexpr size_t kReadSmall = size_t(1) << 13;  // doubles
