@@ -16,7 +16,7 @@
 // is accumulated per walker in FP64 (magnitudes by a log-domain recurrence,
 // so nothing under- or overflows for large N), and reduced per pair at the end.
 //
-// G lanes per walker; positions in shared memory.
+// G lanes per walker on G or G / 2 threads; positions in shared memory.
 // Random numbers: Philox counter {particle, sweep, walker, 2}, init tag 3.
 #include <cuda_runtime.h>
 
@@ -60,47 +60,56 @@ __device__ __forceinline__ double2 cpow_d(double2 z, int k) {
   return r;
 }
 
-// G lanes per walker (one walker group of G consecutive lanes of a warp):
-// lane gl owns the shared particles j = 1 + gl + tG of the Jastrow sums, the
-// estimator's partial products over the same particles and the orbitals
-// l = gl + tG of the estimator; xor-butterfly reductions within the group give
-// every lane bit-identical sums, hence the same accept decision.  Every
-// shuffle sits in control flow that is uniform over the warp (the guide loops
-// run over all kMaxGuideParts slots, the walkers beyond W compute and do not
-// write), so full-warp masks are exact.
+// G lanes per walker on P consecutive threads of a warp, thread gl standing for the
+// V = G / P lanes gl + v P: lane g owns the shared particles j = 1 + g + tG of the
+// Jastrow sums; the estimator's partial products and orbitals and the guide's sums go
+// over the threads.  Xor-butterfly reductions within the group give every thread
+// bit-identical sums, hence the same accept decision.  Every shuffle sits in control
+// flow that is uniform over the warp (the guide loops run over all kMaxGuideParts
+// slots, the walkers beyond W compute and do not write), so full-warp masks are exact.
 constexpr int kOccLanesThreads = 128;
 
-template <int G>
+template <int P>
 __device__ __forceinline__ double group_sum(double v) {
 #pragma unroll
-  for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o, G);
+  for (int o = P / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o, P);
   return v;
 }
 
-template <int G>
-__device__ __forceinline__ float group_sumf(float v) {
+// The FP32 sum over a walker's G lanes held by P threads, thread gl with the V = G / P
+// lanes gl + v P: the butterfly's steps across v come first, in registers, so the sum
+// (and with it the chain of decisions) is the one that G threads form.
+template <int P, int V>
+__device__ __forceinline__ float group_sumf(float (&x)[V]) {
 #pragma unroll
-  for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o, G);
-  return v;
+  for (int h = V / 2; h > 0; h >>= 1)
+#pragma unroll
+    for (int v = 0; v < h; ++v) x[v] += x[v + h];
+  float s = x[0];
+#pragma unroll
+  for (int o = P / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o, P);
+  return s;
 }
 
 // A walker's guide factors: its left row's nL distinct parts and its right row's nR
-// are nL + nR slots, slot s on lane s % G; the lane keeps that part's power sum and
+// are nL + nR slots, slot s on thread s % P; the thread keeps that part's power sum and
 // forms its FP64 log-ratio in every move, and a butterfly adds the terms up.
 //
-// Bound: issue (59 % of the slots with 24 warps an SM, a third of the instructions
-// integer).  With every lane forming all of its walker's terms (two powers and a
-// division each) out of indexed local arrays, N=50 at 65536 walkers took 0.91 ms a
-// sweep, now 0.52.  Keeping the orbital sums in shared memory over the sweeps saves
-// 1 ms of traffic in twenty and costs more in resident blocks (four: 19.1 against
-// 16.7 ms for thirty sweeps).
-template <int G>
-__global__ void __launch_bounds__(kOccLanesThreads, 6) occupation_kernel(const OccArgs a) {
+// Bound: issue (a third of the instructions integer) and the serial part of a move.
+// With every lane forming all of its walker's terms (two powers and a division each) out
+// of indexed local arrays, N=50 at 65536 walkers took 0.91 ms a sweep; with the slots
+// over the lanes 0.52, and with two lanes a thread 0.41.  Five blocks an SM (96 registers)
+// against six: 4.10 and 4.24 ms for ten sweeps.  Keeping the orbital sums in shared
+// memory over the sweeps saves 1 ms of traffic in twenty and costs more in resident
+// blocks (19.1 against 16.7 ms for thirty sweeps, measured with six).
+template <int G, int P>
+__global__ void __launch_bounds__(kOccLanesThreads, 5) occupation_kernel(const OccArgs a) {
   extern __shared__ __align__(16) double occ_smem[];
-  constexpr int WPB = kOccLanesThreads / G;
-  constexpr int SL = (2 * kMaxGuideParts + G - 1) / G;  // slots per lane
+  constexpr int V = G / P;  // lanes of the walker that a thread stands for
+  constexpr int WPB = kOccLanesThreads / P;
+  constexpr int SL = (2 * kMaxGuideParts + P - 1) / P;  // slots per thread
   const int t = threadIdx.x;
-  const int gl = t % G, wl = t / G;
+  const int gl = t % P, wl = t / P;
   const int w = blockIdx.x * WPB + wl;
   const bool live = w < a.W;
   const int N = a.N, NP = a.N + 1;
@@ -120,7 +129,7 @@ __global__ void __launch_bounds__(kOccLanesThreads, 6) occupation_kernel(const O
   double2 gp[SL];
 #pragma unroll
   for (int q = 0; q < SL; ++q) {
-    const int s = gl + q * G;
+    const int s = gl + q * P;
     right[q] = s >= nL;
     const int32_t* part = right[q] ? partsR + 2 * (s - nL) : partsL + 2 * s;
     gk[q] = s < nL + nR ? part[0] : 0;
@@ -132,7 +141,7 @@ __global__ void __launch_bounds__(kOccLanesThreads, 6) occupation_kernel(const O
   const int max_slots = __reduce_max_sync(0xffffffffu, nL + nR);
   // initial positions: uniform in the disk of radius sqrt(2 m N)
   const float r0 = sqrtf(2.f * a.m * N);
-  for (int j = gl; j < NP; j += G) {
+  for (int j = gl; j < NP; j += P) {
     const U4 r = philox4x32_10(U4{uint32_t(j), 0u, uint32_t(w), kTagOccInit}, a.k0, a.k1);
     const float rho = r0 * sqrtf(u01(r.x));
     float sn, cs;
@@ -143,21 +152,25 @@ __global__ void __launch_bounds__(kOccLanesThreads, 6) occupation_kernel(const O
   uint32_t nacc = 0;
   const float sigma = a.sigma;
   const double mm = double(a.m);
-  const int mine = N - 1 > gl ? (N - 2 - gl) / G + 1 : 0;  // shared particles of this lane
+  int mine[V];  // shared particles of each lane
+#pragma unroll
+  for (int v = 0; v < V; ++v)
+    mine[v] = N - 1 > gl + v * P ? (N - 2 - gl - v * P) / G + 1 : 0;
+  const int last = N - 2;  // index of the last shared particle from zs + 1
   // power sums of part q of one side over its particles [j0, j1), to the slot's lane
   auto refresh = [&](int q, int n, const int32_t* parts, int s, int j0, int j1) {
     const int k = q < n ? parts[2 * q] : 0;
     double re = 0.0, im = 0.0;
     if (k > 0)
-      for (int j = j0 + gl; j < j1; j += G) {
+      for (int j = j0 + gl; j < j1; j += P) {
         const double2 v = cpow_d(make_double2(zs[j].x * a.invR, zs[j].y * a.invR), k);
         re += v.x;
         im += v.y;
       }
-    const double2 p = make_double2(group_sum<G>(re), group_sum<G>(im));
+    const double2 p = make_double2(group_sum<P>(re), group_sum<P>(im));
 #pragma unroll
     for (int u = 0; u < SL; ++u)
-      if (q < n && gl + u * G == s) gp[u] = p;
+      if (q < n && gl + u * P == s) gp[u] = p;
   };
   for (int s = 0; s < a.burn + a.sweeps; ++s) {
     // refresh guide power sums: left over 0..N-1, right over 1..N
@@ -167,8 +180,8 @@ __global__ void __launch_bounds__(kOccLanesThreads, 6) occupation_kernel(const O
     double lu_l = 0.0;
     for (int i = 0; i < NP; ++i) {
       // the randoms of move i, Philox {i, sweep, walker, 2}: lane gl draws
-      // those of move i0 + gl for the block of G moves starting at i0
-      if (i % G == 0) {
+      // those of move i0 + gl for the block of P moves starting at i0
+      if (i % P == 0) {
         const U4 r = philox4x32_10(U4{uint32_t(i + gl), uint32_t(s), uint32_t(w), kTagOccMove},
                                    a.k0, a.k1);
         const float rad = sqrtf(-2.f * logf(u01(r.x)));
@@ -178,39 +191,51 @@ __global__ void __launch_bounds__(kOccLanesThreads, 6) occupation_kernel(const O
         dy_l = sigma * (rad * sn);
         lu_l = log(double(u01(r.z)));
       }
-      const float ddx = __shfl_sync(0xffffffffu, dx_l, i % G, G);
-      const float ddy = __shfl_sync(0xffffffffu, dy_l, i % G, G);
-      const double lu = __shfl_sync(0xffffffffu, lu_l, i % G, G);
+      const float ddx = __shfl_sync(0xffffffffu, dx_l, i % P, P);
+      const float ddy = __shfl_sync(0xffffffffu, dy_l, i % P, P);
+      const double lu = __shfl_sync(0xffffffffu, lu_l, i % P, P);
       const float2 zo = zs[i];
       const float2 zn = make_float2(zo.x + ddx, zo.y + ddy);
       // Jastrow log|ratio| over the shared particles 1..N-1 but i: FP32 products of
       // the squared distances, four terms at a time, one log2 per product.  Term u
-      // of the lane is its particle u, or u + 1 from its own particle i on.
-      float lj2 = 0.f;
-      {
-        const int skip = i >= 1 && i < N && (i - 1) % G == gl ? (i - 1) / G : INT_MAX;
-        const int terms = mine - (skip != INT_MAX);
-        const float2* z = zs + 1 + gl;
+      // of a lane is its particle u, or u + 1 from its own particle i on; the terms of
+      // the last, partial product are masked (a factor 1).
+      float lj2[V];
+#pragma unroll
+      for (int v = 0; v < V; ++v) {
+        const int g = gl + v * P;
+        const int skip = i >= 1 && i < N && (i - 1) % G == g ? (i - 1) / G : INT_MAX;
+        const int terms = mine[v] - (skip != INT_MAX);
+        const float2* z = zs + 1;
         float pn = 1.f, po = 1.f;
-        auto term = [&](int u) {
-          const float2 zj = z[(u >= skip ? u + 1 : u) * G];
+        auto factors = [&](float2 zj, float& fn, float& fo) {
           const float dx = zn.x - zj.x, dy = zn.y - zj.y, ex = zo.x - zj.x, ey = zo.y - zj.y;
-          pn *= fmaf(dx, dx, dy * dy);
-          po *= fmaf(ex, ex, ey * ey);
+          fn = fmaf(dx, dx, dy * dy);
+          fo = fmaf(ex, ex, ey * ey);
         };
+        lj2[v] = 0.f;
         int u = 0;
         for (; u + 4 <= terms; u += 4) {
 #pragma unroll
-          for (int v = 0; v < 4; ++v) term(u + v);
-          lj2 += __log2f(pn) - __log2f(po);
+          for (int c = 0; c < 4; ++c) {
+            float fn, fo;
+            factors(z[(u + c) * G + (u + c >= skip ? G + g : g)], fn, fo);
+            pn *= fn;
+            po *= fo;
+          }
+          lj2[v] += __log2f(pn) - __log2f(po);
           pn = po = 1.f;
         }
-        if (u < terms) {
-          for (; u < terms; ++u) term(u);
-          lj2 += __log2f(pn) - __log2f(po);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          float fn, fo;
+          factors(z[min((u + c) * G + (u + c >= skip ? G + g : g), last)], fn, fo);
+          pn *= u + c < terms ? fn : 1.f;
+          po *= u + c < terms ? fo : 1.f;
         }
+        lj2[v] += __log2f(pn) - __log2f(po);
       }
-      const double lj = 0.5 * 0.6931471805599453 * double(group_sumf<G>(lj2));
+      const double lj = 0.5 * 0.6931471805599453 * double(group_sumf<P>(lj2));
       const double gz = double(zo.x) * zo.x + double(zo.y) * zo.y - (double(zn.x) * zn.x + double(zn.y) * zn.y);
       // guide: this lane's log|P'/P| terms of the sides that move (0 moves the left
       // state only, N the right one).  The ratio of squared moduli is formed in FP64,
@@ -223,7 +248,7 @@ __global__ void __launch_bounds__(kOccLanesThreads, 6) occupation_kernel(const O
 #pragma unroll
       for (int q = 0; q < SL; ++q) {
         gn[q] = gp[q];
-        if (q * G < max_slots && gk[q] > 0 && (right[q] ? i > 0 : i < N)) {
+        if (q * P < max_slots && gk[q] > 0 && (right[q] ? i > 0 : i < N)) {
           const double2 p0 = cpow_d(wo, gk[q]), p1 = cpow_d(wn, gk[q]);
           gn[q].x += p1.x - p0.x;
           gn[q].y += p1.y - p0.y;
@@ -232,7 +257,7 @@ __global__ void __launch_bounds__(kOccLanesThreads, 6) occupation_kernel(const O
           gd += 0.5 * 0.6931471805599453 * gr[q] * double(__log2f(float(ratio)));
         }
       }
-      gd = group_sum<G>(gd);
+      gd = group_sum<P>(gd);
       double delta;
       if (i == 0 || i == N) {
         delta = mm * lj + gd + 0.25 * gz;
@@ -272,7 +297,7 @@ __global__ void __launch_bounds__(kOccLanesThreads, 6) occupation_kernel(const O
       }
     };
     int c8 = 0;
-    for (int i = 1 + gl; i < N; i += G) {
+    for (int i = 1 + gl; i < N; i += P) {
       const float2 zi = zs[i];
       const double2 num = make_double2(zi.x - zN.x, zi.y - zN.y);
       const double2 den = make_double2(z0.x - zi.x, z0.y - zi.y);
@@ -281,17 +306,17 @@ __global__ void __launch_bounds__(kOccLanesThreads, 6) occupation_kernel(const O
     }
     unit();
 #pragma unroll
-    for (int o = G / 2; o > 0; o >>= 1)
-      u = cmul(u, make_double2(__shfl_xor_sync(0xffffffffu, u.x, o, G),
-                               __shfl_xor_sync(0xffffffffu, u.y, o, G)));
+    for (int o = P / 2; o > 0; o >>= 1)
+      u = cmul(u, make_double2(__shfl_xor_sync(0xffffffffu, u.x, o, P),
+                               __shfl_xor_sync(0xffffffffu, u.y, o, P)));
     double arg = 0.0;  // arg P_R - arg P_L
 #pragma unroll
     for (int q = 0; q < SL; ++q)
-      if (q * G < max_slots && gk[q] > 0) {
+      if (q * P < max_slots && gk[q] > 0) {
         const double v = gr[q] * atan2(gp[q].y, gp[q].x);
         arg += right[q] ? v : -v;
       }
-    const double phase = group_sum<G>(arg) + mm * atan2(u.y, u.x);
+    const double phase = group_sum<P>(arg) + mm * atan2(u.y, u.x);
     const double2 q0 = make_double2(0.5 * (double(z0.x) * zN.x + double(z0.y) * zN.y),
                                     0.5 * (double(z0.y) * zN.x - double(z0.x) * zN.y));  // z0 conj(zN) / 2
     const double lx = 0.5 * log(q0.x * q0.x + q0.y * q0.y);
@@ -299,11 +324,11 @@ __global__ void __launch_bounds__(kOccLanesThreads, 6) occupation_kernel(const O
     const double base = -0.25 * (double(z0.x) * z0.x + double(z0.y) * z0.y + double(zN.x) * zN.x +
                                  double(zN.y) * zN.y) - log(2.0 * 3.14159265358979323846);
     if (!live) continue;
-    // e^{i (l phi + phase)} by rotations of G phi, one per orbital of the lane
+    // e^{i (l phi + phase)} by rotations of P phi, one per orbital of the lane
     double2 e, rot;
     sincos(gl * phi + phase, &e.y, &e.x);
-    sincos(G * phi, &rot.y, &rot.x);
-    for (int l = gl; l < a.Lc; l += G) {
+    sincos(P * phi, &rot.y, &rot.x);
+    for (int l = gl; l < a.Lc; l += P) {
       // log magnitude of term l: base + l ln|z_0 conj(z_N)/2| - ln l!
       const double la = base + double(l) * lx - lnfact[l];
       if (la > -700.0) {
@@ -325,30 +350,46 @@ int occupation_lanes(int N) {
   return G;
 }
 
-size_t occupation_smem(int N, int Lc) {
-  const int G = occupation_lanes(N);
-  return sizeof(double) * size_t(Lc) + sizeof(float2) * size_t(kOccLanesThreads / G) * (N + 1);
+size_t occupation_smem(int N, int Lc, int threads) {
+  return sizeof(double) * size_t(Lc) + sizeof(float2) * size_t(kOccLanesThreads / threads) * (N + 1);
 }
+size_t occupation_smem(int N, int Lc) { return occupation_smem(N, Lc, occupation_lanes(N)); }
 
-template <int G>
+template <int G, int P>
 int launch_occ_g(const OccArgs& a, cudaStream_t st) {
-  const size_t smem = occupation_smem(a.N, a.Lc);
+  const size_t smem = occupation_smem(a.N, a.Lc, P);
   if (smem > 48 * 1024 &&
-      cudaFuncSetAttribute(occupation_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      cudaFuncSetAttribute(occupation_kernel<G, P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            int(smem)) != cudaSuccess)
     return LEMC_ERR_CUDA;
-  constexpr int WPB = kOccLanesThreads / G;
-  occupation_kernel<G><<<(a.W + WPB - 1) / WPB, kOccLanesThreads, smem, st>>>(a);
+  constexpr int WPB = kOccLanesThreads / P;
+  occupation_kernel<G, P><<<(a.W + WPB - 1) / WPB, kOccLanesThreads, smem, st>>>(a);
   return cudaPeekAtLastError() == cudaSuccess ? LEMC_OK : LEMC_ERR_CUDA;
+}
+
+// A thread stands for two of a walker's lanes from eight lanes on, where the halved
+// warps still fill fifteen of an SM's twenty places and a block's positions leave room for
+// five: what a warp does once per move is then shared by twice the walkers.  Ten sweeps,
+// one lane -> two lanes a thread, ms: N=50, 65536 walkers 4.99 -> 4.10; 20000 (17 warps
+// an SM) 1.76 -> 1.61; N=90, 30000 7.02 -> 5.35; but N=60, 7000 (6 warps) 0.92 -> 1.33.
+// Four lanes a thread lose the overlap of the lanes' products (N=50: 6.4), and of four
+// lanes two a thread lose too (N=20: 1.45 -> 1.82).
+constexpr int kOccMinWarps = 15, kOccSMs = 148;
+template <int G>
+int launch_occ_lanes(const OccArgs& a, cudaStream_t st) {
+  constexpr int P = G >= 8 ? G / 2 : G;
+  if (int64_t(a.W) * P / 32 >= kOccMinWarps * kOccSMs && occupation_smem(a.N, a.Lc, P) <= 40 * 1024)
+    return launch_occ_g<G, P>(a, st);
+  return launch_occ_g<G, G>(a, st);
 }
 
 int launch_occupation(const OccArgs& a, cudaStream_t st) {
   if (occupation_smem(a.N, a.Lc) > 227 * 1024) return LEMC_ERR_CAPACITY;
   switch (occupation_lanes(a.N)) {
-    case 4: return launch_occ_g<4>(a, st);
-    case 8: return launch_occ_g<8>(a, st);
-    case 16: return launch_occ_g<16>(a, st);
-    default: return launch_occ_g<32>(a, st);
+    case 4: return launch_occ_lanes<4>(a, st);
+    case 8: return launch_occ_lanes<8>(a, st);
+    case 16: return launch_occ_lanes<16>(a, st);
+    default: return launch_occ_lanes<32>(a, st);
   }
 }
 
