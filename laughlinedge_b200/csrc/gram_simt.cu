@@ -25,16 +25,21 @@ constexpr size_t kGramSmem = 40 * 1024;
 // TA TB / 4 threads and the block holds NG = 1024 / (TA TB) groups that share
 // each staged chunk of walkers, summed at the end.
 //
-// Bound: the FP64 pipe (64 FMA/cycle/SM).  A (pair, walker) costs 10 FMAs: 4
-// for conj(a) b, 6 for the three weighted sums (folding the weights into one
-// operand first would cost 12).  The staged values are widened to FP64 once per
-// chunk; widening inside the product loop, seven conversions for every 10 FMAs
-// at a quarter of their rate, and one output per thread held the previous
-// 16 x 16 form at 5 % of the pipe.  The small shapes keep the padding of small
-// sectors low and spread their walkers over more blocks.
+// Bound: the FP64 pipe (64 FMA/cycle/SM; 65 % busy), with the shared-memory loads of the
+// operands beside it.  A (pair, walker) costs 10 FMAs: 4 for conj(a) b, 6 for the three
+// weighted sums (folding the weights into one operand first would cost 12).  The staged
+// values are widened to FP64 once per chunk; widening inside the product loop, seven
+// conversions for every 10 FMAs at a quarter of their rate, and one output per thread
+// held the previous 16 x 16 form at 5 % of the pipe.  A thread stages a value's two
+// components together (one 16-byte store instead of two of 8, half the index work: 2.96
+// -> 2.77 ms for 526 states at 65536 walkers, and 2.70 with four walkers in flight).  4 x 2
+// outputs a thread save a third of the loads but leave one block an SM, 2.91 ms.  The
+// small shapes keep the padding of small sectors low and spread their walkers over more
+// blocks.
 //
-// Measured (B200): cross planes of 526 states at 65536 walkers (N=100, dL
-// 0,2..16) @CROSS@; 29 states (N=8, dL 1..6) at 4096 walkers @SMALL@.
+// Measured (B200): Gram of 526 states (N=100, dL 0,2..16) at 65536 walkers 2.70 ms, their
+// cross planes 8.3 ms (40.3 in the 16 x 16 form); 29 states (N=8, dL 1..6) at 4096
+// walkers 21 us (101).
 template <int TA, int TB>
 struct Tile {
   static constexpr int TX = TB / 2, TY = TA / 2;  // threads: tx over b, ty over a
@@ -42,10 +47,10 @@ struct Tile {
   static constexpr int NG = kGramThreads / TPG;
   static constexpr int CH = TA == 8 ? (TB == 8 ? 128 : TB == 16 ? 64 : 32) : (TB == 16 ? 64 : 32);
   static constexpr int SA = TA + 1, SB = TB + 1;  // double2 row strides per walker
-  static constexpr int NF = 2 * (TA + TB) * CH / kGramThreads;  // staged floats per thread
+  static constexpr int NF = (TA + TB) * CH / kGramThreads;  // staged values per thread
   static constexpr size_t kStage = sizeof(double2) * CH * (SA + SB) + sizeof(double) * 3 * CH;
   static constexpr size_t kReduce = NG > 1 ? sizeof(double) * (NG / 2) * TPG * 24 : 0;
-  static_assert(NF * kGramThreads == 2 * (TA + TB) * CH && CH % 32 == 0 && CH % NG == 0, "tile shape");
+  static_assert(NF * kGramThreads == (TA + TB) * CH && CH % 32 == 0 && CH % NG == 0, "tile shape");
   static_assert(kStage <= kGramSmem && kReduce <= kGramSmem, "tile shape");
 };
 
@@ -61,25 +66,27 @@ __device__ __forceinline__ void gram_tile(const float* __restrict__ V, int ldv,
   double* wt = reinterpret_cast<double*>(sb + T::CH * T::SB);  // [3][CH]
   const int tid = threadIdx.x;
   const int g = tid / T::TPG, tg = tid % T::TPG;
-  const int tx = tg % T::TX, ty = tg / T::TX;
+  // 16 threads over b: a warp takes 8 of them by 4 over a, whose 16-byte loads read fewer
+  // distinct rows than 16 by 2
+  constexpr bool kSquare = T::TX == 16;
+  const int tx = kSquare ? (tg & 7) + ((tg >> 5) & 1) * 8 : tg % T::TX;
+  const int ty = kSquare ? ((tg >> 3) & 3) + (tg >> 6) * 4 : tg / T::TX;
 
-  // staged element e = it * 256 + tid: walker e % CH, tile row e / CH in the
-  // order Re a, Im a, Re b, Im b (a warp reads 32 consecutive walkers of a row)
-  float pf[T::NF];
+  // staged element e = it * 256 + tid: walker e % CH of tile row e / CH, the rows of a
+  // first (a warp reads 32 consecutive walkers of a row)
+  float2 pf[T::NF];
   float pw[3] = {0.f, 0.f, 0.f};
   auto fetch = [&](int c0) {
 #pragma unroll
     for (int it = 0; it < T::NF; ++it) {
       const int e = it * kGramThreads + tid;
       const int s = e % T::CH, q = e / T::CH;
-      const bool isb = q >= 2 * TA;
-      const int t = isb ? q - 2 * TA : q;
-      const int tw = isb ? TB : TA;
-      const int r = (isb ? jb.b0 : jb.a0) + (t >= tw ? t - tw : t);
+      const bool isb = q >= TA;
+      const int r = isb ? jb.b0 + q - TA : jb.a0 + q;
       const int dim = isb ? jb.Db : jb.Da;
-      const int row = (isb ? jb.row_b : jb.row_a) + (t >= tw ? dim : 0) + r;
-      const int wi = c0 + s;
-      pf[it] = (wi < wend && r < dim) ? V[(size_t)row * ldv + wi] : 0.f;
+      const float* v = V + (size_t)((isb ? jb.row_b : jb.row_a) + r) * ldv + c0 + s;
+      const bool in = c0 + s < wend && r < dim;
+      pf[it] = in ? make_float2(v[0], v[(size_t)dim * ldv]) : make_float2(0.f, 0.f);
     }
     if (tid < T::CH) {
       const int wi = c0 + tid;
@@ -93,16 +100,11 @@ __device__ __forceinline__ void gram_tile(const float* __restrict__ V, int ldv,
     }
   };
   auto stage = [&]() {
-    double* da = reinterpret_cast<double*>(sa);
-    double* db = reinterpret_cast<double*>(sb);
 #pragma unroll
     for (int it = 0; it < T::NF; ++it) {
       const int e = it * kGramThreads + tid;
       const int s = e % T::CH, q = e / T::CH;
-      if (q < 2 * TA)
-        da[2 * (s * T::SA + (q % TA)) + (q / TA)] = double(pf[it]);
-      else
-        db[2 * (s * T::SB + ((q - 2 * TA) % TB)) + (q - 2 * TA) / TB] = double(pf[it]);
+      (q < TA ? sa[s * T::SA + q] : sb[s * T::SB + q - TA]) = make_double2(pf[it].x, pf[it].y);
     }
     if (tid < T::CH) {
 #pragma unroll
@@ -124,7 +126,7 @@ __device__ __forceinline__ void gram_tile(const float* __restrict__ V, int ldv,
     stage();
     __syncthreads();
     if (c0 + T::CH < wend) fetch(c0 + T::CH);  // lands while this chunk is summed
-#pragma unroll 2
+#pragma unroll 4
     for (int s = g; s < T::CH; s += T::NG) {
       double2 a[2], b[2];
 #pragma unroll
@@ -299,8 +301,8 @@ int launch_gram_simt(const float* V, int ldv, const float* rec_w, int ldw, int W
                      cudaStream_t st) {
   if (n_jobs <= 0) return LEMC_OK;
   // Walker split: about sixteen blocks for each of the 2 x 148 resident slots, so
-  // the last wave is a small share (526 states:
-  // 9.2 ms; with six blocks a slot 9.9 ms), in whole
+  // the last wave is a small share (cross planes of 526 states,
+  // before the paired staging: 9.2 ms; with six blocks a slot 9.9 ms), in whole
   // 128-walker chunks; every split costs one FP64 atomic per output and plane.
   const long want = (16L * 2 * 148 + n_jobs - 1) / n_jobs;
   const int chunks = (W + 127) / 128;
