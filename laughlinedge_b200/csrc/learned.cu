@@ -649,7 +649,7 @@ es_objective_kernel(const float2* __restrict__ cfgs, int n_cfg, int N, float inv
 }
 
 // ES gradient (ascent on J) and one Adam step; the BF16 copy follows the
-// FP32 master weights.  trace[step] = mean J over all perturbations.
+// FP32 master weights.  *trace = mean J over all perturbations (trace may be null).
 // kAdamLanes threads share a parameter's sum over the pairs (a thread alone runs
 // pairs Philox draws in a row on 19 blocks: 11 us; now 4.5).
 constexpr int kAdamLanes = 8;
@@ -660,10 +660,10 @@ es_adam_kernel(float* __restrict__ theta, float* __restrict__ am,
                float lr, uint32_t step, uint32_t k0, uint32_t k1,
                double* __restrict__ trace) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t == 0) {
+  if (t == 0 && trace) {
     double s = 0.0;
     for (int p = 0; p < 2 * pairs; ++p) s += J[p];
-    trace[step] = s / (2.0 * pairs * batch);
+    *trace = s / (2.0 * pairs * batch);
   }
   const int k = t / kAdamLanes, part = t % kAdamLanes;
   double g = 0.0;
@@ -895,7 +895,10 @@ extern "C" int lemc_proposal_train(lemc_proposal* p, const void* configs, int n_
   if (p->trace_cap < tc->steps) {
     cudaFree(p->trace);
     p->trace = nullptr;
-    if (cudaMalloc(&p->trace, sizeof(double) * tc->steps) != cudaSuccess) return LEMC_ERR_CUDA;
+    p->trace_cap = 0;
+    if (cudaMalloc(&p->trace, sizeof(double) * tc->steps) != cudaSuccess ||
+        cudaMemset(p->trace, 0, sizeof(double) * tc->steps) != cudaSuccess)
+      return LEMC_ERR_CUDA;
     p->trace_cap = tc->steps;
   }
   const uint32_t k0 = uint32_t(tc->seed), k1 = uint32_t(tc->seed >> 32);
@@ -910,9 +913,13 @@ extern "C" int lemc_proposal_train(lemc_proposal* p, const void* configs, int n_
           static_cast<const float2*>(configs), n_cfg, N, p->invR, float(p->m), p->theta, tc->es_sigma,
           step, k0, k1, tc->batch, p->J);
     });
+    // Entry s + step of the trace, where it has one: with step counted from the
+    // weights' last reset, a first call's entry 2 s holds step s.
+    const uint64_t at = uint64_t(s) + step;
     es_adam_kernel<<<(kNParams * kAdamLanes + 255) / 256, 256>>>(p->theta, p->am, p->av, p->wts, p->J,
                                                     tc->pairs, tc->batch, tc->es_sigma, tc->lr,
-                                                    step, k0, k1, p->trace + s);
+                                                    step, k0, k1,
+                                                    at < uint64_t(p->trace_cap) ? p->trace + at : nullptr);
     if (cudaPeekAtLastError() != cudaSuccess) return LEMC_ERR_CUDA;
     ++p->train_steps;
   }
