@@ -74,6 +74,8 @@ constexpr uint32_t kTagLearned = 4u, kTagTrain = 5u, kTagEs = 6u;
 constexpr int kWarpsPerBlock = 4;   // sampler / evaluation blocks
 constexpr int kSweepBlocks = 8;     // resident sweep blocks per SM
 constexpr int kTrainBlocks = 592;   // ES blocks of a step: four per SM
+constexpr int kMaxDirections = 512; // perturbation directions formed at a time (19 KB each)
+constexpr int kMaxSamples = 32768;  // training samples formed at a time (384 bytes each)
 constexpr int kTrainWarps = 16;     // ES blocks share one perturbed weight set
 constexpr float kLn2 = 0.6931471805599453f;
 
@@ -199,21 +201,18 @@ __device__ __noinline__ uint32_t nearest_full(const float2* zs, int N, int self,
   return pop_nearest<S, S>(key, min(kNbr, N - 1), lane, lost);
 }
 
-// The network at centre zc for particle `self` of the walker whose positions
-// are zs[0..N), from the lane's keys about zc.  All 32 lanes call it; every lane
-// returns the same values.  P holds the parameters in their shared-memory slots
-// (p_slot); gbuf is the warp's shared scratch of kH floats.
+// The rotation into the local (radial, tangential) frame of zc.
+__device__ __forceinline__ float2 local_frame(float2 zc, float r2) {
+  if (!(r2 > 1e-20f)) return make_float2(1.f, 0.f);
+  const float ri = rsqrtf(r2);
+  return make_float2(zc.x * ri, zc.y * ri);
+}
+
+// Frame coordinates of the lane's neighbour of zc (lane < min(kNbr, N - 1)), from the
+// lane's keys about zc; the other lanes' value is unspecified.
 template <int S>
-__device__ __forceinline__ NetOut net_eval(const float* __restrict__ P, const float2* zs, int N,
-                                           int self, float2 zc, float invR, int lane, float* gbuf,
-                                           uint32_t (&key)[S]) {
-  const float r2 = zc.x * zc.x + zc.y * zc.y;
-  float c = 1.f, s = 0.f;
-  if (r2 > 1e-20f) {
-    const float ri = rsqrtf(r2);
-    c = zc.x * ri;
-    s = zc.y * ri;
-  }
+__device__ __forceinline__ float2 neighbour(const float2* zs, int N, int self, float2 zc, float2 frame,
+                                            int lane, uint32_t (&key)[S]) {
   static_assert(kNbr <= 32, "one neighbour per lane");
   constexpr int kDepth = S > 4 ? 4 : S;
   const int cnt = min(kNbr, N - 1);
@@ -223,16 +222,34 @@ __device__ __forceinline__ NetOut net_eval(const float* __restrict__ P, const fl
   if constexpr (kDepth < S) {
     if (lost) mine = nearest_full<S>(zs, N, self, zc, lane);  // warp-uniform
   }
+  if (lane >= cnt) return make_float2(0.f, 0.f);
+  const int j = int(mine & 0xFFu);
+  const float dx = zs[j].x - zc.x, dy = zs[j].y - zc.y;
+  const float xr = (dx * frame.x + dy * frame.y) * kInScale;
+  const float xt = (dy * frame.x - dx * frame.y) * kInScale;
+  return make_float2(xr, xt);
+}
+
+// The network at centre zc for particle `self` of the walker whose positions
+// are zs[0..N), from the lane's keys about zc, or from its neighbours' frame
+// coordinates where they are given.  All 32 lanes call it; every lane
+// returns the same values.  P holds the parameters in their shared-memory slots
+// (p_slot); gbuf is the warp's shared scratch of kH floats.
+template <int S>
+__device__ __forceinline__ NetOut net_eval(const float* __restrict__ P, const float2* zs, int N,
+                                           int self, float2 zc, float invR, int lane, float* gbuf,
+                                           uint32_t (&key)[S], const float2* given = nullptr) {
+  const float r2 = zc.x * zc.x + zc.y * zc.y;
+  const int cnt = min(kNbr, N - 1);
   // each lane forms the frame coordinates of its own neighbour once; phi then
   // runs over the neighbours in the same ascending order, two hidden units per lane
   // as one packed pair
   float2* nb = reinterpret_cast<float2*>(gbuf);
-  if (lane < cnt) {
-    const int j = int(mine & 0xFFu);
-    const float dx = zs[j].x - zc.x, dy = zs[j].y - zc.y;
-    const float xr = (dx * c + dy * s) * kInScale;
-    const float xt = (dy * c - dx * s) * kInScale;
-    nb[lane] = make_float2(xr, xt);
+  if (given) {
+    if (lane < cnt) nb[lane] = given[lane];
+  } else {
+    const float2 x = neighbour<S>(zs, N, self, zc, local_frame(zc, r2), lane, key);
+    if (lane < cnt) nb[lane] = x;
   }
   __syncwarp();
   const float2 W0X = make_float2(P[kOffW1 + 2 * lane], P[kOffW1 + 2 * (lane + 32)]);
@@ -294,6 +311,13 @@ struct Move {
   float2 zn;       // proposed position
   float log_a;     // natural log of the Metropolis-Hastings ratio
   float jump2;     // |z' - z|^2
+};
+
+// What a training sample's configuration gives all perturbations alike: the frame
+// coordinates of the 16 nearest about z_i and each lane's products of squared distances.
+struct Sample {
+  float2 nb[kNbr];
+  float po[2][32];
 };
 
 // The forward half of a move: the network at z_i, the proposed position, and
@@ -368,15 +392,22 @@ __device__ __forceinline__ float reverse_log_density(const NetOut& b, float2 zo,
 template <int S, class Wanted>
 __device__ __forceinline__ bool move_step(const float* __restrict__ P, const float2* zs, int N, int i,
                                           float invR, float m, float e_r, float e_t, int lane,
-                                          float* gbuf, Forward& fw, float& lq, Wanted&& wanted) {
+                                          float* gbuf, Forward& fw, float& lq, Wanted&& wanted,
+                                          const Sample* given = nullptr) {
   const float2 zo = zs[i];
   float2 zc = zo;
   float po[2];
   uint32_t key[S];
-  make_keys<S>(zs, N, i, zo, lane, key, po);
+  if (given) {
+#pragma unroll
+    for (int q = 0; q < (S + 3) / 4; ++q) po[q] = given->po[q][lane];
+  } else {
+    make_keys<S>(zs, N, i, zo, lane, key, po);
+  }
 #pragma unroll 1
   for (int pass = 0; pass < 2; ++pass) {
-    const NetOut net = net_eval<S>(P, zs, N, i, zc, invR, lane, gbuf, key);
+    const NetOut net = net_eval<S>(P, zs, N, i, zc, invR, lane, gbuf, key,
+                                   pass == 0 && given ? given->nb : nullptr);
     if (pass == 0) {
       fw = propose_forward<S>(net, zs, N, i, zo, po, m, e_r, e_t, lane, key);
       zc = fw.zn;
@@ -391,10 +422,11 @@ __device__ __forceinline__ bool move_step(const float* __restrict__ P, const flo
 template <int S>
 __device__ __forceinline__ Move propose(const float* __restrict__ P, const float2* zs, int N, int i,
                                         float invR, float m, float e_r, float e_t, int lane,
-                                        float* gbuf) {
+                                        float* gbuf, const Sample* given = nullptr) {
   Forward fw;
   float lq = 0.f;
-  move_step<S>(P, zs, N, i, invR, m, e_r, e_t, lane, gbuf, fw, lq, [](const Forward&) { return true; });
+  move_step<S>(P, zs, N, i, invR, m, e_r, e_t, lane, gbuf, fw, lq, [](const Forward&) { return true; },
+               given);
   Move mv;
   mv.zn = fw.zn;
   mv.log_a = fw.part + lq;
@@ -597,19 +629,67 @@ learned_eval_kernel(const float2* __restrict__ cfgs, int n, int N, float invR, f
   }
 }
 
+// Direction `pair` of a step's perturbations, parameter k.
+__device__ __forceinline__ float es_noise(int k, int pair, uint32_t step, uint32_t k0, uint32_t k1) {
+  const U4 r = philox4x32_10(U4{uint32_t(k), uint32_t(pair), step, kTagEs}, k0, k1);
+  float e0, e1;
+  box_muller(r.x, r.y, e0, e1);
+  return e0;
+}
+
+// The directions of `steps` steps from `step0` on, [step][pair][parameter].
+__global__ void __launch_bounds__(256)
+es_noise_kernel(uint32_t step0, int steps, int pairs, uint32_t k0, uint32_t k1,
+                float* __restrict__ noise) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= steps * pairs * kNParams) return;
+  const int k = e % kNParams, q = e / kNParams;
+  noise[e] = es_noise(k, q % pairs, step0 + uint32_t(q / pairs), k0, k1);
+}
+
+// Samples first .. first + count of the run that starts at step `step0`, `batch` a step:
+// a warp each.
+template <int S>
+__global__ void __launch_bounds__(kWarpsPerBlock * 32)
+es_samples_kernel(const float2* __restrict__ cfgs, int n_cfg, int N, uint32_t step0, uint32_t k0,
+                  uint32_t k1, int first, int batch, int count, Sample* __restrict__ samples) {
+  extern __shared__ float2 zsm[];
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const int q = blockIdx.x * kWarpsPerBlock + wib;
+  if (q >= count) return;
+  const int g = first + q;
+  const U4 r = philox4x32_10(U4{uint32_t(g % batch), step0 + uint32_t(g / batch), 0u, kTagTrain}, k0, k1);
+  const int c = int(r.x % uint32_t(n_cfg)), i = int(r.y % uint32_t(N));
+  float2* zs = zsm + size_t(wib) * N;
+  for (int j = lane; j < N; j += 32) zs[j] = cfgs[size_t(c) * N + j];
+  __syncwarp();
+  const float2 zo = zs[i];
+  uint32_t key[S];
+  float po[2];
+  make_keys<S>(zs, N, i, zo, lane, key, po);
+#pragma unroll
+  for (int v = 0; v < (S + 3) / 4; ++v) samples[q].po[v][lane] = po[v];
+  const float2 x = neighbour<S>(zs, N, i, zo, local_frame(zo, zo.x * zo.x + zo.y * zo.y), lane, key);
+  if (lane < kNbr) samples[q].nb[lane] = x;
+}
+
 // ES objective: the blocks (x, pert) share the batch of a perturbation, each
 // evaluating kTrainWarps samples at a time with the parameters
 // theta + sign * sigma * e_pair; J[pert] += sum of min(1, A) |dz|^2.
-// Forming the kNParams perturbed parameters (Philox and Box-Muller each) costs a
-// block about what its samples cost once, so a block takes as many rounds of
-// samples as leave about four blocks per SM (launch below): with one round
-// each, 307 us a step at 64 perturbations of 1024 samples (N=200); now 171 us (two
-// blocks per SM 174, eight 191).
+// A block takes as many rounds of samples as leave about four blocks per SM (launch
+// below): with one round each, the parameters cost a block as much as its samples, 307 us
+// a step at 64 perturbations of 1024 samples (N=200); now 152 us (two blocks per SM 158,
+// eight 166).  What does not depend on the block is formed ahead: the directions e_pair
+// (es_noise_kernel; up to kMaxDirections, more are formed by each block) and what the
+// network at z_i reads of a sample's configuration, the same for every perturbation
+// (es_samples_kernel).  Without the first 162 us, without either 171; the two launches
+// cost 1.8 us a step.  Bound: latency, 32 warps an SM (64 registers).
 template <int S>
 __global__ void __launch_bounds__(kTrainWarps * 32)
 es_objective_kernel(const float2* __restrict__ cfgs, int n_cfg, int N, float invR, float m,
                     const float* __restrict__ theta, float es_sigma, uint32_t step, uint32_t k0,
-                    uint32_t k1, int batch, double* __restrict__ J) {
+                    uint32_t k1, int first, int batch, const Sample* __restrict__ samples,
+                    const float* __restrict__ noise, double* __restrict__ J) {
   __shared__ __align__(16) float P[kNParams];
   __shared__ __align__(16) float gsm[kTrainWarps][kH];
   __shared__ double part[kTrainWarps];
@@ -618,24 +698,22 @@ es_objective_kernel(const float2* __restrict__ cfgs, int n_cfg, int N, float inv
   const int pair = pert >> 1;
   const float sgn = (pert & 1) ? -es_sigma : es_sigma;
   for (int k = threadIdx.x; k < kNParams; k += blockDim.x) {
-    const U4 r = philox4x32_10(U4{uint32_t(k), uint32_t(pair), step, kTagEs}, k0, k1);
-    float e0, e1;
-    box_muller(r.x, r.y, e0, e1);
+    const float e0 = noise ? noise[size_t(pair) * kNParams + k] : es_noise(k, pair, step, k0, k1);
     P[p_slot(k)] = theta[k] + sgn * e0;
   }
   __syncthreads();
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   float2* zs = zsm + size_t(wib) * N;
   double sum = 0.0;
-  for (int sidx = blockIdx.x * kTrainWarps + wib; sidx < batch; sidx += gridDim.x * kTrainWarps) {
-    const U4 r = philox4x32_10(U4{uint32_t(sidx), step, 0u, kTagTrain}, k0, k1);
+  for (int q = blockIdx.x * kTrainWarps + wib; q < batch; q += gridDim.x * kTrainWarps) {
+    const U4 r = philox4x32_10(U4{uint32_t(first + q), step, 0u, kTagTrain}, k0, k1);
     const int c = int(r.x % uint32_t(n_cfg)), i = int(r.y % uint32_t(N));
     __syncwarp();  // the previous sample's positions are read
     for (int j = lane; j < N; j += 32) zs[j] = cfgs[size_t(c) * N + j];
     __syncwarp();
     float er, et;
     box_muller(r.z, r.w, er, et);
-    const Move mv = propose<S>(P, zs, N, i, invR, m, er, et, lane, gsm[wib]);
+    const Move mv = propose<S>(P, zs, N, i, invR, m, er, et, lane, gsm[wib], samples + q);
     const float val = (mv.log_a >= 0.f ? 1.f : __expf(mv.log_a)) * mv.jump2;
     if (val == val) sum += val;
   }
@@ -651,14 +729,14 @@ es_objective_kernel(const float2* __restrict__ cfgs, int n_cfg, int N, float inv
 // ES gradient (ascent on J) and one Adam step; the BF16 copy follows the
 // FP32 master weights.  *trace = mean J over all perturbations (trace may be null).
 // kAdamLanes threads share a parameter's sum over the pairs (a thread alone runs
-// pairs Philox draws in a row on 19 blocks: 11 us; now 4.5).
+// pairs Philox draws in a row on 19 blocks: 11 us; with eight 4.8, with the directions read 2.9).
 constexpr int kAdamLanes = 8;
 __global__ void __launch_bounds__(256)
 es_adam_kernel(float* __restrict__ theta, float* __restrict__ am,
                float* __restrict__ av, __nv_bfloat16* __restrict__ wts,
                const double* __restrict__ J, int pairs, int batch, float es_sigma,
                float lr, uint32_t step, uint32_t k0, uint32_t k1,
-               double* __restrict__ trace) {
+               const float* __restrict__ noise, double* __restrict__ trace) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t == 0 && trace) {
     double s = 0.0;
@@ -668,9 +746,8 @@ es_adam_kernel(float* __restrict__ theta, float* __restrict__ am,
   const int k = t / kAdamLanes, part = t % kAdamLanes;
   double g = 0.0;
   for (int p = part; p < pairs; p += kAdamLanes) {
-    const U4 r = philox4x32_10(U4{uint32_t(k), uint32_t(p), step, kTagEs}, k0, k1);
-    float e0, e1;
-    box_muller(r.x, r.y, e0, e1);
+    if (k >= kNParams) break;
+    const float e0 = noise ? noise[size_t(p) * kNParams + k] : es_noise(k, p, step, k0, k1);
     g += (J[2 * p] - J[2 * p + 1]) * double(e0);
   }
 #pragma unroll
@@ -740,6 +817,10 @@ struct lemc_proposal {
   int J_cap = 0;
   double* trace = nullptr;
   int trace_cap = 0;
+  Sample* samples = nullptr;    // training samples ahead
+  int samples_cap = 0;
+  float* noise = nullptr;       // perturbation directions ahead
+  int noise_cap = 0;            // of this many (step, pair)s
   uint64_t train_steps = 0;     // Adam steps taken (bias correction, Philox counters)
 };
 
@@ -813,6 +894,8 @@ extern "C" int lemc_proposal_destroy(lemc_proposal* p) {
   cudaFree(p->wts);
   cudaFree(p->J);
   cudaFree(p->trace);
+  cudaFree(p->samples);
+  cudaFree(p->noise);
   delete p;
   return LEMC_OK;
 }
@@ -901,24 +984,67 @@ extern "C" int lemc_proposal_train(lemc_proposal* p, const void* configs, int n_
       return LEMC_ERR_CUDA;
     p->trace_cap = tc->steps;
   }
+  // the samples of several steps, or a part of one step's, at a time: 12 MB at most,
+  // kept with the proposal like the directions' 10 MB
+  const int64_t all = int64_t(tc->steps) * tc->batch;
+  const int part = std::min(tc->batch, kMaxSamples);         // of one step
+  const int ahead = std::max(1, std::min(tc->steps, kMaxSamples / tc->batch));  // steps
+  const int cap = int(std::min<int64_t>(all, int64_t(ahead) * part));
+  if (p->samples_cap < cap) {
+    cudaFree(p->samples);
+    p->samples = nullptr;
+    p->samples_cap = 0;
+    if (cudaMalloc(&p->samples, sizeof(Sample) * cap) != cudaSuccess) return LEMC_ERR_CUDA;
+    p->samples_cap = cap;
+  }
+  // directions of as many steps, or none (each block forms its own) if one step has more
+  const int dirs = std::min(tc->steps, kMaxDirections / tc->pairs);
+  if (p->noise_cap < dirs * tc->pairs) {
+    cudaFree(p->noise);
+    p->noise = nullptr;
+    p->noise_cap = 0;
+    if (cudaMalloc(&p->noise, sizeof(float) * size_t(dirs) * tc->pairs * kNParams) != cudaSuccess)
+      return LEMC_ERR_CUDA;
+    p->noise_cap = dirs * tc->pairs;
+  }
   const uint32_t k0 = uint32_t(tc->seed), k1 = uint32_t(tc->seed >> 32);
-  const int rounds = (tc->batch + kTrainWarps - 1) / kTrainWarps;
   const int perts = 2 * tc->pairs;
-  const dim3 grid(std::min(rounds, std::max(1, kTrainBlocks / perts)), perts);
+  const float2* cfgs = static_cast<const float2*>(configs);
   for (int s = 0; s < tc->steps; ++s) {
     const uint32_t step = uint32_t(p->train_steps);
     if (cudaMemsetAsync(p->J, 0, sizeof(double) * 2 * tc->pairs) != cudaSuccess) return LEMC_ERR_CUDA;
-    with_slots(N, [&](auto sl) {
-      es_objective_kernel<sl.value><<<grid, kTrainWarps * 32, walker_smem(N, kTrainWarps)>>>(
-          static_cast<const float2*>(configs), n_cfg, N, p->invR, float(p->m), p->theta, tc->es_sigma,
-          step, k0, k1, tc->batch, p->J);
-    });
+    const float* noise = nullptr;
+    if (dirs > 0) {
+      if (s % dirs == 0) {
+        const int n = std::min(dirs, tc->steps - s);
+        es_noise_kernel<<<(n * tc->pairs * kNParams + 255) / 256, 256>>>(step, n, tc->pairs, k0, k1,
+                                                                         p->noise);
+      }
+      noise = p->noise + size_t(s % dirs) * tc->pairs * kNParams;
+    }
+    for (int64_t begin = 0; begin < tc->batch; begin += part) {
+      const int first = int(begin);
+      const int n = std::min(part, tc->batch - first);  // of this step in this launch
+      const int rounds = (n + kTrainWarps - 1) / kTrainWarps;
+      const dim3 grid(std::min(rounds, std::max(1, kTrainBlocks / perts)), perts);
+      with_slots(N, [&](auto sl) {
+        if (s % ahead == 0) {
+          const int count = part < tc->batch ? n : std::min(ahead, tc->steps - s) * tc->batch;
+          es_samples_kernel<sl.value><<<(count + kWarpsPerBlock - 1) / kWarpsPerBlock,
+                                        kWarpsPerBlock * 32, walker_smem(N)>>>(
+              cfgs, n_cfg, N, step, k0, k1, first, tc->batch, count, p->samples);
+        }
+        es_objective_kernel<sl.value><<<grid, kTrainWarps * 32, walker_smem(N, kTrainWarps)>>>(
+            cfgs, n_cfg, N, p->invR, float(p->m), p->theta, tc->es_sigma, step, k0, k1, first, n,
+            p->samples + size_t(s % ahead) * part, noise, p->J);
+      });
+    }
     // Entry s + step of the trace, where it has one: with step counted from the
     // weights' last reset, a first call's entry 2 s holds step s.
     const uint64_t at = uint64_t(s) + step;
     es_adam_kernel<<<(kNParams * kAdamLanes + 255) / 256, 256>>>(p->theta, p->am, p->av, p->wts, p->J,
                                                     tc->pairs, tc->batch, tc->es_sigma, tc->lr,
-                                                    step, k0, k1,
+                                                    step, k0, k1, noise,
                                                     at < uint64_t(p->trace_cap) ? p->trace + at : nullptr);
     if (cudaPeekAtLastError() != cudaSuccess) return LEMC_ERR_CUDA;
     ++p->train_steps;
