@@ -364,7 +364,6 @@ def rooflines(L, w, mode, t_sweep, t_basis, t_gram, learned, clocks, reverse=1.0
     flop_gram = W * 8.0 * 3 * sd2
     traffic = traffic_from_profiles()
     tag = w["workload"]
-    tf32_peak = peaks["bf16_tflops"] / 2.0 if mode == L._lib.GRAM_TF32X3 else peaks["bf16_tflops"]
     roofs = {
         "sweep": {"bound": "fp32", "achieved": flop_sweep / (t_sweep * 1e-3) / 1e12,
                   "peak": fp32_peak, "unit": "TFLOP/s",
@@ -377,9 +376,9 @@ def rooflines(L, w, mode, t_sweep, t_basis, t_gram, learned, clocks, reverse=1.0
                   "kernel": "basis_kernel", "traffic": traffic.get("basis@" + tag),
                   "ms_per_launch": t_basis},
         "gram": {"bound": "tensor", "achieved": flop_gram / (t_gram * 1e-3) / 1e12,
-                 "peak": tf32_peak, "unit": "TFLOP/s",
-                 "peak_source": (f"{peak_kind} bf16_tflops / 2 (dense TF32 rate)" if mode == L._lib.GRAM_TF32X3
-                                 else f"{peak_kind} bf16_tflops"),
+                 "peak": peaks["bf16_tflops"], "unit": "TFLOP/s",
+                 # 16-bit operand terms in every mode (FP16 for tf32x3)
+                 "peak_source": f"{peak_kind} bf16_tflops",
                  "kernel": "gram_tc_kernel", "traffic": traffic.get("gram@" + tag),
                  "ms_per_launch": t_gram},
     }
