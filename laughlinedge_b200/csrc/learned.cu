@@ -72,7 +72,12 @@ constexpr int kMaxN = 256;                 // packed kNN keys carry 8 index bits
 constexpr int kMaxSlots = kMaxN / 32;      // most particles per lane
 constexpr uint32_t kTagLearned = 4u, kTagTrain = 5u, kTagEs = 6u;
 constexpr int kWarpsPerBlock = 4;   // sampler / evaluation blocks
-constexpr int kSweepBlocks = 8;     // resident sweep blocks per SM
+// Resident sweep blocks per SM: seven leave 72 registers, room for the held parameters.
+// Four sweeps at N=200, 65536 walkers: nothing held 71.1 ms with eight blocks, 72.5 with
+// seven; held, 68.7 with seven, 70.8 with six; a part of them 69.6 to 72.0; records of W2
+// too, 71.8 (two, five blocks) to 75.1 (ten, four).  With the four output sums in one
+// butterfly (head_sums) 67.0.
+constexpr int kSweepBlocks = 7;
 constexpr int kTrainBlocks = 592;   // ES blocks of a step: four per SM
 constexpr int kMaxDirections = 512; // perturbation directions formed at a time (19 KB each)
 constexpr int kMaxSamples = 32768;  // training samples formed at a time (384 bytes each)
@@ -130,6 +135,21 @@ __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
+}
+
+// warp_sum of four values at once: the first two steps of the butterfly hand half of the
+// values over each, so ten shuffles do for twenty; the same pairs are added.
+__device__ __forceinline__ void head_sums(float (&o)[4], int lane) {
+  const bool h16 = lane & 16, h8 = lane & 8;
+  float a = h16 ? o[2] : o[0], b = h16 ? o[3] : o[1];
+  a += __shfl_xor_sync(0xffffffffu, h16 ? o[0] : o[2], 16);
+  b += __shfl_xor_sync(0xffffffffu, h16 ? o[1] : o[3], 16);
+  float s = h8 ? b : a;
+  s += __shfl_xor_sync(0xffffffffu, h8 ? a : b, 8);
+#pragma unroll
+  for (int d = 4; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) o[q] = __shfl_sync(0xffffffffu, s, 8 * q);
 }
 
 // Squared distance of slot t's particle from zc, and whether the lane has one
@@ -230,13 +250,30 @@ __device__ __forceinline__ float2 neighbour(const float2* zs, int N, int self, f
   return make_float2(xr, xt);
 }
 
+// Parameters that a lane keeps in registers over its moves: the words of hidden units
+// lane, lane + 32 outside W2.  The shared-memory pipe is the busiest unit (80 %), a move
+// reads them once per network evaluation, and a word costs a register here against a
+// load each time; W2's records, four words a load, do not pay (see kSweepBlocks).
+struct Held {
+  float2 w1x, w1y, b1, w2r, b2, w3[4];
+  __device__ __forceinline__ Held(const float* P, int lane) {
+    w1x = make_float2(P[kOffW1 + 2 * lane], P[kOffW1 + 2 * (lane + 32)]);
+    w1y = make_float2(P[kOffW1 + 2 * lane + 1], P[kOffW1 + 2 * (lane + 32) + 1]);
+    b1 = make_float2(P[kOffB1 + lane], P[kOffB1 + lane + 32]);
+    w2r = make_float2(P[kOffW2 + kW2Packed + lane], P[kOffW2 + kW2Packed + lane + 32]);
+    b2 = make_float2(P[kOffB2 + lane], P[kOffB2 + lane + 32]);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) w3[q] = make_float2(P[kOffW3 + q * kH + lane], P[kOffW3 + q * kH + lane + 32]);
+  }
+};
+
 // The network at centre zc for particle `self` of the walker whose positions
 // are zs[0..N), from the lane's keys about zc, or from its neighbours' frame
 // coordinates where they are given.  All 32 lanes call it; every lane
 // returns the same values.  P holds the parameters in their shared-memory slots
 // (p_slot); gbuf is the warp's shared scratch of kH floats.
 template <int S>
-__device__ __forceinline__ NetOut net_eval(const float* __restrict__ P, const float2* zs, int N,
+__device__ __forceinline__ NetOut net_eval(const Held& held, const float* __restrict__ P, const float2* zs, int N,
                                            int self, float2 zc, float invR, int lane, float* gbuf,
                                            uint32_t (&key)[S], const float2* given = nullptr) {
   const float r2 = zc.x * zc.x + zc.y * zc.y;
@@ -252,19 +289,16 @@ __device__ __forceinline__ NetOut net_eval(const float* __restrict__ P, const fl
     if (lane < cnt) nb[lane] = x;
   }
   __syncwarp();
-  const float2 W0X = make_float2(P[kOffW1 + 2 * lane], P[kOffW1 + 2 * (lane + 32)]);
-  const float2 W0Y = make_float2(P[kOffW1 + 2 * lane + 1], P[kOffW1 + 2 * (lane + 32) + 1]);
-  const float2 B0 = make_float2(P[kOffB1 + lane], P[kOffB1 + lane + 32]);
   float2 g = make_float2(0.f, 0.f);
 #pragma unroll
   for (int n = 0; n < kNbr; n += 2) {
     const float4 x = reinterpret_cast<const float4*>(nb)[n / 2];
     if (S > 1 || n < cnt) {
-      const float2 h = __ffma2_rn(W0X, make_float2(x.x, x.x), __ffma2_rn(W0Y, make_float2(x.y, x.y), B0));
+      const float2 h = __ffma2_rn(held.w1x, make_float2(x.x, x.x), __ffma2_rn(held.w1y, make_float2(x.y, x.y), held.b1));
       g = __fadd2_rn(g, make_float2(fmaxf(h.x, 0.f), fmaxf(h.y, 0.f)));
     }
     if (S > 1 || n + 1 < cnt) {
-      const float2 h = __ffma2_rn(W0X, make_float2(x.z, x.z), __ffma2_rn(W0Y, make_float2(x.w, x.w), B0));
+      const float2 h = __ffma2_rn(held.w1x, make_float2(x.z, x.z), __ffma2_rn(held.w1y, make_float2(x.w, x.w), held.b1));
       g = __fadd2_rn(g, make_float2(fmaxf(h.x, 0.f), fmaxf(h.y, 0.f)));
     }
   }
@@ -281,8 +315,7 @@ __device__ __forceinline__ NetOut net_eval(const float* __restrict__ P, const fl
   __syncwarp();
   const float4* G4 = reinterpret_cast<const float4*>(gbuf);
   const float4* W4 = reinterpret_cast<const float4*>(P + kOffW2) + lane;
-  float2 kk = make_float2(fmaf(P[kOffW2 + kW2Packed + lane], sf, P[kOffB2 + lane]),
-                          fmaf(P[kOffW2 + kW2Packed + lane + 32], sf, P[kOffB2 + lane + 32]));
+  float2 kk = make_float2(fmaf(held.w2r.x, sf, held.b2.x), fmaf(held.w2r.y, sf, held.b2.y));
   auto rho_in = [&](int v, float ga, float gb) {
     const float4 w = W4[v * 32];
     kk = __ffma2_rn(make_float2(w.z, w.w), make_float2(gb, gb), kk);
@@ -299,9 +332,10 @@ __device__ __forceinline__ NetOut net_eval(const float* __restrict__ P, const fl
   const float k0 = fmaxf(kk.x, 0.f), k1 = fmaxf(kk.y, 0.f);
   float o[4];
 #pragma unroll
-  for (int q = 0; q < 4; ++q)
-    o[q] = warp_sum(fmaf(P[kOffW3 + q * kH + lane], k0, P[kOffW3 + q * kH + lane + 32] * k1)) +
-           P[kOffB3 + q];
+  for (int q = 0; q < 4; ++q) o[q] = fmaf(held.w3[q].x, k0, held.w3[q].y * k1);
+  head_sums(o, lane);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) o[q] += P[kOffB3 + q];
   return NetOut{o[0], o[1], fminf(fmaxf(o[2], kLogSMin), kLogSMax),
                 fminf(fmaxf(o[3], kLogSMin), kLogSMax)};
 }
@@ -390,7 +424,7 @@ __device__ __forceinline__ float reverse_log_density(const NetOut& b, float2 zo,
 // (a rolled loop), which leaves the instruction cache room for its loops unrolled:
 // a copy each took 73.0 ms for four sweeps at N=200, W=65536, this 72.0.
 template <int S, class Wanted>
-__device__ __forceinline__ bool move_step(const float* __restrict__ P, const float2* zs, int N, int i,
+__device__ __forceinline__ bool move_step(const Held& held, const float* __restrict__ P, const float2* zs, int N, int i,
                                           float invR, float m, float e_r, float e_t, int lane,
                                           float* gbuf, Forward& fw, float& lq, Wanted&& wanted,
                                           const Sample* given = nullptr) {
@@ -406,7 +440,7 @@ __device__ __forceinline__ bool move_step(const float* __restrict__ P, const flo
   }
 #pragma unroll 1
   for (int pass = 0; pass < 2; ++pass) {
-    const NetOut net = net_eval<S>(P, zs, N, i, zc, invR, lane, gbuf, key,
+    const NetOut net = net_eval<S>(held, P, zs, N, i, zc, invR, lane, gbuf, key,
                                    pass == 0 && given ? given->nb : nullptr);
     if (pass == 0) {
       fw = propose_forward<S>(net, zs, N, i, zo, po, m, e_r, e_t, lane, key);
@@ -420,12 +454,12 @@ __device__ __forceinline__ bool move_step(const float* __restrict__ P, const flo
 }
 
 template <int S>
-__device__ __forceinline__ Move propose(const float* __restrict__ P, const float2* zs, int N, int i,
+__device__ __forceinline__ Move propose(const Held& held, const float* __restrict__ P, const float2* zs, int N, int i,
                                         float invR, float m, float e_r, float e_t, int lane,
                                         float* gbuf, const Sample* given = nullptr) {
   Forward fw;
   float lq = 0.f;
-  move_step<S>(P, zs, N, i, invR, m, e_r, e_t, lane, gbuf, fw, lq, [](const Forward&) { return true; },
+  move_step<S>(held, P, zs, N, i, invR, m, e_r, e_t, lane, gbuf, fw, lq, [](const Forward&) { return true; },
                given);
   Move mv;
   mv.zn = fw.zn;
@@ -548,6 +582,7 @@ learned_sweep_kernel(const SweepArgs a, const __nv_bfloat16* __restrict__ wts) {
   __syncthreads();
   if (!live) return;
   __syncwarp();
+  const Held held(P, lane);
   const uint32_t sweep_base = a.sweep0 + (a.sweep_ctr ? *a.sweep_ctr : 0u);
   const float m = float(a.m);
   uint32_t nacc = 0, nrev = 0;
@@ -572,7 +607,7 @@ learned_sweep_kernel(const SweepArgs a, const __nv_bfloat16* __restrict__ wts) {
       Forward fw;
       float lq = 0.f;
       bool acc = false;
-      if (move_step<S>(P, zs, N, i, a.invR, m, er, et, lane, gsm[wib], fw, lq,
+      if (move_step<S>(held, P, zs, N, i, a.invR, m, er, et, lane, gsm[wib], fw, lq,
                        [&](const Forward& f) { return lu < f.part + kLogQbMax; })) {
         acc = lu < fw.part + lq;
         ++nrev;
@@ -614,8 +649,9 @@ learned_eval_kernel(const float2* __restrict__ cfgs, int n, int N, float invR, f
   uint32_t key[S];
   float po[2];
   make_keys<S>(zs, N, i, zs[i], lane, key, po);
-  const NetOut f = net_eval<S>(P, zs, N, i, zs[i], invR, lane, gsm[wib], key);
-  const Move mv = propose<S>(P, zs, N, i, invR, m, eps[2 * sidx], eps[2 * sidx + 1], lane, gsm[wib]);
+  const Held held(P, lane);
+  const NetOut f = net_eval<S>(held, P, zs, N, i, zs[i], invR, lane, gsm[wib], key);
+  const Move mv = propose<S>(held, P, zs, N, i, invR, m, eps[2 * sidx], eps[2 * sidx + 1], lane, gsm[wib]);
   if (lane == 0) {
     float* o = out + size_t(sidx) * 8;
     o[0] = f.mr;
@@ -703,6 +739,7 @@ es_objective_kernel(const float2* __restrict__ cfgs, int n_cfg, int N, float inv
   }
   __syncthreads();
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const Held held(P, lane);
   float2* zs = zsm + size_t(wib) * N;
   double sum = 0.0;
   for (int q = blockIdx.x * kTrainWarps + wib; q < batch; q += gridDim.x * kTrainWarps) {
@@ -713,7 +750,7 @@ es_objective_kernel(const float2* __restrict__ cfgs, int n_cfg, int N, float inv
     __syncwarp();
     float er, et;
     box_muller(r.z, r.w, er, et);
-    const Move mv = propose<S>(P, zs, N, i, invR, m, er, et, lane, gsm[wib], samples + q);
+    const Move mv = propose<S>(held, P, zs, N, i, invR, m, er, et, lane, gsm[wib], samples + q);
     const float val = (mv.log_a >= 0.f ? 1.f : __expf(mv.log_a)) * mv.jump2;
     if (val == val) sum += val;
   }
