@@ -942,6 +942,11 @@ int lemc_set_sectors(lemc_ctx* c, const int32_t* sectors, int n) {
   c->gram_plane = goff;
   LEMC_TRY(build_jobs(c));
   LEMC_TRY(c->gram.alloc(6 * c->gram_plane));
+  // The read-back block of the largest sector: growing it from sector to sector freed and
+  // allocated up to twenty times in a first read, 5 ms and now and then 100 (each free waits
+  // for the device).  Where there is no room for it, a read takes what it needs.
+  const size_t largest = *std::max_element(c->basis.sector_dim.begin(), c->basis.sector_dim.end());
+  if (c->d_read.alloc(2 * kReadHead + 6 * largest * largest) != LEMC_OK) cudaGetLastError();
   LEMC_TRY(build_program(c));
   LEMC_TRY(alloc_records(c));
   c->row_scale.assign(c->D, 1.0);
