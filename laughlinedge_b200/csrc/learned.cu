@@ -422,7 +422,7 @@ __device__ __forceinline__ float reverse_log_density(const NetOut& b, float2 zo,
 // says so, the network at the proposed configuration; lq is ln q(z | z') then, and
 // the result whether it was formed.  Both networks run through one copy of the code
 // (a rolled loop), which leaves the instruction cache room for its loops unrolled:
-// a copy each took 73.0 ms for four sweeps at N=200, W=65536, this 72.0.
+// a copy each took 73.0 ms for four sweeps at N=200, W=65536, this 72.0 (67.0 now).
 template <int S, class Wanted>
 __device__ __forceinline__ bool move_step(const Held& held, const float* __restrict__ P, const float2* zs, int N, int i,
                                           float invR, float m, float e_r, float e_t, int lane,
@@ -714,8 +714,8 @@ es_samples_kernel(const float2* __restrict__ cfgs, int n_cfg, int N, uint32_t st
 // theta + sign * sigma * e_pair; J[pert] += sum of min(1, A) |dz|^2.
 // A block takes as many rounds of samples as leave about four blocks per SM (launch
 // below): with one round each, the parameters cost a block as much as its samples, 307 us
-// a step at 64 perturbations of 1024 samples (N=200); now 152 us (two blocks per SM 158,
-// eight 166).  What does not depend on the block is formed ahead: the directions e_pair
+// a step at 64 perturbations of 1024 samples (N=200); now 147 us (152, two blocks per SM
+// 158, eight 166 before a lane held its parameters).  What does not depend on the block is formed ahead: the directions e_pair
 // (es_noise_kernel; up to kMaxDirections, more are formed by each block) and what the
 // network at z_i reads of a sample's configuration, the same for every perturbation
 // (es_samples_kernel).  Without the first 162 us, without either 171; the two launches
