@@ -251,7 +251,7 @@ __device__ __forceinline__ float2 neighbour(const float2* zs, int N, int self, f
 }
 
 // Parameters that a lane keeps in registers over its moves: the words of hidden units
-// lane, lane + 32 outside W2.  The shared-memory pipe is the busiest unit (80 %), a move
+// lane, lane + 32 outside W2.  The shared-memory pipe is the busiest unit (80 %, now 76), a move
 // reads them once per network evaluation, and a word costs a register here against a
 // load each time; W2's records, four words a load, do not pay (see kSweepBlocks).
 struct Held {
